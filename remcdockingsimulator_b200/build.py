@@ -14,6 +14,7 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -93,8 +94,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
     objdir = os.path.join(LIBDIR, "obj")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
-    for src in sources():
+
+    def compile_one(src: str) -> str:
         obj = os.path.join(objdir, os.path.basename(src)[:-3] + ".o")
         cmd = [NVCC] + ARCH + FLAGS + ["-c", src, "-o", obj]
         if verbose:
@@ -104,7 +105,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("nvcc failed for %s:\n%s%s" % (src, r.stdout, r.stderr))
         if verbose:
             sys.stderr.write(r.stderr)
-        objs.append(obj)
+        return obj
+
+    with ThreadPoolExecutor() as pool:
+        objs = list(pool.map(compile_one, sources()))
     tmp = LIB + ".tmp"
     cmd = [NVCC] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)

@@ -159,6 +159,18 @@ __device__ __forceinline__ float crowd_energy(float r2, float A, float cut2) {
   return e;
 }
 
+// Change of a crowder pair's energy from squared distance ro to rn: the new
+// energy's last product enters the difference unrounded (written out, so that
+// every caller rounds alike).
+template <bool R12, bool CUT>
+__device__ __forceinline__ float crowd_change(float rn, float ro, float A, float cut2) {
+  if (CUT)
+    return __fsub_rn(crowd_energy<R12, true>(rn, A, cut2), crowd_energy<R12, true>(ro, A, cut2));
+  const float in2 = fast_rcp(rn), in6 = in2 * in2 * in2;
+  const float eo = crowd_energy<R12, false>(ro, A, cut2);
+  return R12 ? __fmaf_rn(A * in6, in6, -eo) : __fmaf_rn(A, in6, -eo);
+}
+
 __device__ __forceinline__ float pair_r2(float4 a, float4 b, float L, float invL) {
   float dx = min_image(a.x - b.x, L, invL);
   float dy = min_image(a.y - b.y, L, invL);
@@ -246,10 +258,24 @@ __device__ __forceinline__ float2 crowd_energy2(float2 r2, float2 A, float2 cut2
   return e;
 }
 
+// crowd_change for two pairs
+template <bool R12, bool CUT>
+__device__ __forceinline__ float2 crowd_change2(float2 rn, float2 ro, float2 A, float2 cut2) {
+  if (CUT) {
+    const float2 en = crowd_energy2<R12, true>(rn, A, cut2), eo = crowd_energy2<R12, true>(ro, A, cut2);
+    return __fadd2_rn(en, make_float2(-eo.x, -eo.y));
+  }
+  const float2 in2 = make_float2(fast_rcp(rn.x), fast_rcp(rn.y));
+  const float2 in6 = __fmul2_rn(__fmul2_rn(in2, in2), in2);
+  const float2 eo = crowd_energy2<R12, false>(ro, A, cut2);
+  const float2 t = R12 ? __fmul2_rn(A, in6) : A;
+  return __ffma2_rn(t, in6, make_float2(-eo.x, -eo.y));
+}
+
 // Kim-Hummer + Debye-Hueckel energy of two residue pairs that share the table
 // entry T (the moved bead's new and old position against one bead j), in
-// packed FP32: pair_energy_r2's operations for a residue pair, each product
-// and sum rounded on its own.
+// packed FP32: pair_energy_r2's operations for a residue pair, with the last
+// product unrounded in the sum.
 __device__ __forceinline__ float2 kh_energy2(float2 r2, float4 T, float c_xi) {
   const float2 rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
   const float2 rinv2 = __fmul2_rn(rinv, rinv);
@@ -264,8 +290,7 @@ __device__ __forceinline__ float2 kh_energy2(float2 r2, float4 T, float c_xi) {
   const float2 r = __fmul2_rn(r2, rinv);
   const float2 arg = __fmul2_rn(r, make_float2(c_xi, c_xi));
   const float2 ex = make_float2(fast_ex2(arg.x), fast_ex2(arg.y));
-  const float2 dh = __fmul2_rn(__fmul2_rn(make_float2(T.w, T.w), ex), rinv);
-  return __fadd2_rn(lj, dh);
+  return __ffma2_rn(__fmul2_rn(make_float2(T.w, T.w), ex), rinv, lj);
 }
 
 // ---------------------------------------------------------------- moves
@@ -328,7 +353,7 @@ __device__ __forceinline__ void quat_mul(double qw, double qx, double qy, double
 // For x in [0, 3L) the result is x, x - L or x - 2L, and each subtraction is
 // exact (Sterbenz: y/2 <= x <= 2y), so this equals fmodf bit for bit; other
 // inputs (centres placed outside the box) take fmodf itself.
-__device__ __forceinline__ float wrap_box(float x, float L) {
+static __device__ __noinline__ float wrap_box(float x, float L) {  // rarely called: out of the way
   if (x >= 0.0f) {
     if (x < L) return x;
     const float L2 = 2.0f * L;  // exact

@@ -24,7 +24,6 @@
 //                      CudaFunctions.cu:455-685).
 //   exchange_kernel    one warp per system, disjoint temperature pairs in
 //                      parallel lanes (main.cpp:1427-1453).
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -39,6 +38,7 @@
 
 #include "remc_device.cuh"
 #include "remc_internal.h"
+#include "remc_sweep.cuh"
 
 using namespace remc;
 
@@ -68,37 +68,6 @@ int set_error(int code, const char* fmt, ...) {
     if (_e != cudaSuccess)                                                               \
       return set_error(REMC_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e));   \
   } while (0)
-
-struct SysDev {
-  int n_beads, n_mol, n_rep, lmax;
-  int inst0, bead_base, mol_base, mstart_off;
-  float box, invbox;
-  int translate_only_crowders;
-  int n_chain_beads;  // beads of residue type; the rest are crowders
-  int crowd_type;     // the one bead type of every crowder, or -1 (none or mixed)
-  // 1: every bead pair is within 1.5 box lengths on each axis, for the state
-  // uploaded last and every state the sweep can reach from it (set on the
-  // device by fold_flag_kernel at each upload; the sweep then folds the
-  // minimum image)
-  int fold_mi;
-};
-
-// Per-step proposal record: everything about step s of one replica that does
-// not depend on the replica's state (Philox draws, chosen molecule, move type,
-// translation vector, step quaternion). Written by proposal_kernel for a
-// whole sweep, streamed through shared memory by sweep_kernel.
-struct StepRec {
-  double q[4];      // step quaternion (rotation)
-  double thr;       // Metropolis threshold -log(u)/beta: accept iff dE < thr
-  float t[3];       // translation vector
-  int m;            // molecule
-  int m0;           // its first bead
-  int info;         // bits 0-29: its bead count; bit 30: rotation; bit 31: crowder
-};
-constexpr int kRecRotate = 1 << 30;
-constexpr int kRecCrowd = (int)(1u << 31);
-constexpr int kRecCount = kRecRotate - 1;
-static_assert(sizeof(StepRec) == 64, "StepRec layout");
 
 struct ProposalArgs {
   const SysDev* sys;
@@ -210,713 +179,6 @@ __global__ void __launch_bounds__(256) rank_kernel(const long long* __restrict__
   }
   rank = __reduce_add_sync(0xffffffffu, rank);
   if (lane == 0) order[rank] = i;
-}
-
-// A bound conformation recorded by Replica::sample (Replica.cpp:1717-1780):
-// header + one pose (rotation quaternion, centre) per molecule.
-struct SampleHeader {
-  int inst;
-  uint32_t label;     // step label (start of the sampling chunk, main.cpp:983-987)
-  double e_nc;        // potential + chain-chain pair energy (the sample() sum)
-  double e;           // potential
-  float temperature;
-  int n_mol;
-  uint32_t pose_offset;
-  int pad;
-};
-struct SamplePose {
-  double q[4];
-  float c[3];
-  float pad;
-};
-
-struct SweepArgs {
-  const SysDev* sys;
-  const int* inst_sys;
-  const int* inst_list;  // instances, largest expected cost first
-  int* queue;            // work counter (persistent grid), or null: CTA b runs inst_list[b]
-  int n_list;
-  float4* pos;
-  float4* rel;
-  float4* centre;
-  double* quat;
-  const int* mol_start;
-  const float4* tab;
-  const StepRec* recs;   // [n_inst][rec_stride]
-  double* energy;
-  double* ecc;           // chain-chain part of the energy (sample() sum)
-  const int* temp_idx;
-  const float* ladder;
-  // sampling (Replica::sample): every `sample_every` steps, labels from step0
-  int sample_every;
-  uint32_t sample_after;
-  double bound_thr;
-  const uint32_t* ctrl;
-  uint32_t step0;
-  int* n_samples;
-  int* n_bound;
-  SampleHeader* sample_out;
-  SamplePose* pose_out;
-  unsigned* sample_cursor;  // [0] records, [1] poses, [2] dropped
-  unsigned sample_cap, pose_cap;
-  int* acc_neg;          // accepted with dE < 0
-  int* acc_boltz;        // accepted by the Boltzmann test
-  int* rej;
-  unsigned long long* evals_kh;     // residue-residue pair evaluations
-  unsigned long long* evals_crowd;  // pair evaluations involving a crowder
-  int rec_stride, rec_offset;       // records of step s at rec_offset + s
-  int n_steps;
-  int nmax, mmax, lmax;  // shared-memory capacities
-  int mol_in_smem;       // centres resident in shared memory
-  int csize;             // CTAs per replica (a thread-block cluster), 1, 2, 4 or 8
-  // beads kept in global memory (systems too large for shared memory): trial
-  // positions and trial relative positions of each (instance, CTA rank), 6 lmax
-  float4* trial_scratch;
-  EnergyConsts K;
-};
-
-constexpr int kRing = 64;  // proposal records held in shared memory (two halves)
-
-// Shared-memory layout of sweep_kernel, in bytes, for capacities (nmax beads,
-// mmax molecules, lmax beads per molecule).
-struct SweepSmem {
-  size_t tab, beads, centres, trial_pos, trial_rel, ring, red, total;
-  static __host__ __device__ size_t take(size_t& off, size_t bytes) {
-    size_t o = off;
-    off += (bytes + 15) & ~size_t(15);
-    return o;
-  }
-  // mol_in_smem = 0: molecule centres and starts stay in global memory (the
-  // largest systems), everything else as usual. beads_in_smem = 0: the beads
-  // and the trial buffers stay in global memory too (systems of any size)
-  static __host__ __device__ SweepSmem make(int nmax, int mmax, int lmax, int mol_in_smem,
-                                            int csize = 1, int beads_in_smem = 1) {
-    SweepSmem s;
-    size_t off = 0;
-    s.tab = take(off, sizeof(float4) * kNT * kNT);
-    s.beads = take(off, beads_in_smem ? sizeof(float4) * nmax : 0);
-    s.centres = take(off, mol_in_smem ? sizeof(float4) * mmax : 0);
-    s.trial_pos = take(off, beads_in_smem ? sizeof(float4) * 4 * lmax : 0);
-    s.trial_rel = take(off, beads_in_smem ? sizeof(float4) * 2 * lmax : 0);
-    s.ring = take(off, sizeof(StepRec) * kRing);
-    s.red = take(off, sizeof(double) * 2 * csize * 2 * 32);  // [parity][rank][dE, dcc][warp]
-    s.total = off;
-    return s;
-  }
-};
-
-// Sum of 8 FP64 partials (16-byte aligned) in a fixed pairwise order; the
-// entries of warps a smaller CTA does not have hold an exact zero. Every
-// thread evaluates it and gets the same value.
-__device__ __forceinline__ double tree_sum8(const double* v) {
-  const double2* v2 = reinterpret_cast<const double2*>(v);
-  const double2 a = v2[0], b = v2[1], c = v2[2], d = v2[3];
-  return ((a.x + a.y) + (b.x + b.y)) + ((c.x + c.y) + (d.x + d.y));
-}
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n"); }
-
-// One CTA per replica-instance, persistent over the sweep. The instance's beads
-// and molecule centres stay in shared memory for all n_steps steps.
-//
-// Ownership: in the pair loop thread t reads only beads j = t (mod T), and the
-// same thread writes those beads when a move is accepted, so bead updates need
-// no barrier. Every thread computes the FP64 sum of the per-warp partials and
-// the Metropolis decision itself (same order, same result), and tracks the
-// previous step's move to read a molecule moved one step ago from registers or
-// the trial buffer rather than from another thread's not-yet-ordered write.
-// A step of a one-bead molecule therefore costs one barrier; a chain step
-// costs two (trial positions are built by the owners of the chain's beads).
-// GB: the beads stay where they are in global memory (updated in place, no
-// prologue copy and no write-back) and the trial buffers live in per-instance
-// global scratch; every access pattern, owner and barrier is the same as with
-// the beads in shared memory (a CTA barrier orders global memory for the CTA,
-// a cluster barrier for the cluster; the CTAs of a cluster write identical
-// values to the beads they own).
-template <bool R12, bool CUT, bool CLUSTER, bool GB>
-__global__ void __launch_bounds__(256, 2) sweep_kernel(SweepArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const SweepSmem L = SweepSmem::make(A.nmax, A.mmax, A.lmax, A.mol_in_smem, A.csize, !GB);
-  float4* s_tab = reinterpret_cast<float4*>(smem_raw + L.tab);
-  float4* const sm_beads = reinterpret_cast<float4*>(smem_raw + L.beads);
-  float4* s_cent = reinterpret_cast<float4*>(smem_raw + L.centres);
-  float4* const sm_tpos = reinterpret_cast<float4*>(smem_raw + L.trial_pos);
-  StepRec* s_ring = reinterpret_cast<StepRec*>(smem_raw + L.ring);
-  double* s_red = reinterpret_cast<double*>(smem_raw + L.red);
-
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int tmask = nthr - 1;  // nthr is a power of two
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-  // A replica may span a cluster of csize CTAs: every CTA holds the whole
-  // replica and runs every step, the pair loops split bead j over the
-  // cluster's threads (CTA rank r, thread t takes j = r T + t mod csize T;
-  // within a CTA that is still j = t mod T, so ownership is unchanged), the
-  // warps' partial sums go to every CTA's shared memory, and one cluster
-  // barrier per step replaces the CTA barrier. Rank 0 alone writes state that
-  // is not idempotent (rotations, counters, samples) and the final state.
-  const int csize = CLUSTER ? A.csize : 1;
-  const int crank = CLUSTER ? (int)cooperative_groups::this_cluster().block_rank() : 0;
-  const int gtid = crank * nthr + tid, gstride = nthr * csize, gmask = gstride - 1;
-  __shared__ int s_next;
-  for (int it = 0;; ++it) {
-  int idx;
-  if (A.queue) {
-    if (tid == 0) s_next = atomicAdd(A.queue, 1);
-    __syncthreads();
-    idx = s_next;
-    __syncthreads();  // every thread has read s_next before it is rewritten
-    if (idx >= A.n_list) break;
-  } else {
-    if (it > 0) break;
-    idx = blockIdx.x / csize;
-  }
-  const int inst = A.inst_list[idx];
-  const int sysid = A.inst_sys[inst];
-  const SysDev S = A.sys[sysid];
-  const int slot = inst - S.inst0;
-  const int N = S.n_beads, M = S.n_mol;
-  const int bead_off = S.bead_base + slot * N;
-  const int mol_off = S.mol_base + slot * M;
-  const float box = S.box, invbox = S.invbox;
-  const StepRec* recs = A.recs + (size_t)inst * A.rec_stride + A.rec_offset;
-  const int n_steps = A.n_steps;
-  float4* const s_beads = GB ? A.pos + bead_off : sm_beads;
-  // per-(instance, CTA rank) global scratch of 6 lmax entries: trial
-  // positions (used when the beads stay in global memory) and trial
-  // relative positions
-  float4* const scratch =
-      A.trial_scratch + ((size_t)inst * csize + crank) * 6 * (size_t)A.lmax;
-  // trial positions of a chain move, two entries per moved bead k, by step
-  // parity b: s_tpos[2 (b lmax + k)] = (new x, old x, new y, old y),
-  // s_tpos[2 (b lmax + k) + 1] = (new z, old z, meta word, table row offset),
-  // so that each (new, old) coordinate pair is a register pair of the packed
-  // pair loops as loaded
-  float4* const s_tpos = GB ? scratch : sm_tpos;
-  // rotated relative positions of the chain's beads, computed with its trial
-  // positions by the beads' owners and installed by the same threads (each
-  // thread reads back only what it wrote), in shared memory, or in global
-  // scratch when the beads stay in global memory. The install writes rel
-  // without reading it, so the CTAs of a cluster, which all install the same
-  // values, cannot read one another's update. Two buffers by step parity,
-  // like the trial positions: the next step's owners (another molecule,
-  // other threads) write theirs before any barrier, while slower warps may
-  // still install from this step's
-  float4* const s_trel =
-      GB ? scratch + 4 * (size_t)A.lmax : reinterpret_cast<float4*>(smem_raw + L.trial_rel);
-
-  // ---- prologue: make the instance resident in shared memory
-  for (int i = tid; i < kNT * kNT; i += nthr) s_tab[i] = A.tab[i];
-  // partial-sum entries of warps this CTA does not have: an exact zero
-  for (int i = tid; i < 2 * csize * 2 * 8; i += nthr)
-    if ((i & 7) >= nwarps) s_red[(i >> 3) * 32 + (i & 7)] = 0.0;
-  if (!GB)
-    for (int i = tid; i < N; i += nthr) s_beads[i] = A.pos[bead_off + i];
-  // molecule centres: shared memory, or global memory for the largest
-  // systems (thread 0 writes a centre; others read it only after a later
-  // barrier, which orders global memory within the CTA as well)
-  float4* cent = A.mol_in_smem ? s_cent : A.centre + mol_off;
-  if (A.mol_in_smem)
-    for (int i = tid; i < M; i += nthr) s_cent[i] = A.centre[mol_off + i];
-  {
-    // first ring fill: records of steps 0..min(kRing, n_steps)-1, 16 B per copy
-    const int nrec = min(kRing, n_steps);
-    const int chunks = nrec * (int)(sizeof(StepRec) / 16);
-    for (int c = tid; c < chunks; c += nthr)
-      cp_async16(reinterpret_cast<char*>(s_ring) + 16 * c,
-                 reinterpret_cast<const char*>(recs) + 16 * c);
-    cp_async_commit();
-    cp_async_wait_all();
-  }
-  // every thread keeps the running energies (all see the same dE and decision)
-  double energy = A.energy[inst], ecc = A.ecc[inst];
-  int n_neg = 0, n_boltz = 0, n_rej = 0, n_samp = 0, n_bnd = 0;
-  unsigned long long ev_kh = 0, ev_crowd = 0;
-  const int ncb = S.n_chain_beads;  // beads [0, ncb) belong to chains
-  const int ctype = S.crowd_type;   // the crowders' one type, or -1
-  const uint32_t step0 = A.ctrl ? A.ctrl[0] : A.step0;
-  int to_sample = A.sample_every;  // steps left in the current sampling chunk
-  __shared__ long long s_pose_slot;
-  // every CTA of a cluster has started before any writes another's shared memory
-  if (CLUSTER)
-    cooperative_groups::this_cluster().sync();
-  else
-    __syncthreads();
-  float4 next_c = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (n_steps > 0 && !A.mol_in_smem) next_c = cent[s_ring[0].m];
-
-  // previous step, known to every thread
-  int p_m = -1, p_acc = 0, p_rot = 0, p_n = 0, p_b = 0;
-  float4 p_single = make_float4(0.f, 0.f, 0.f, 0.f);  // accepted one-bead position
-  float p_nc0 = 0.f, p_nc1 = 0.f, p_nc2 = 0.f;          // accepted new centre
-
-  for (int s = 0; s < n_steps; ++s) {
-    // ---- prefetch the next ring half (records s+31 .. s+62). The half it
-    // overwrites ends with step s-2's record, which is read until after step
-    // s-2's barrier; a thread at step s has passed step s-1's barrier, so no
-    // thread reads it any more
-    if ((s & 31) == 1 && s > 1 && s + 31 < n_steps) {
-      const int first = s + 31;
-      const int nrec = min(32, n_steps - first);
-      const int chunks = nrec * (int)(sizeof(StepRec) / 16);
-      char* dst = reinterpret_cast<char*>(s_ring + (first & (kRing - 1)));
-      const char* src = reinterpret_cast<const char*>(recs + first);
-      for (int c = tid; c < chunks; c += nthr) cp_async16(dst + 16 * c, src + 16 * c);
-      cp_async_commit();
-    }
-    const StepRec& recs_ = s_ring[s & (kRing - 1)];  // stable for the whole step
-    struct {
-      int m, rotate, crowd;
-      float t[3];
-    } rec;
-    rec.m = recs_.m;
-    rec.rotate = (recs_.info & kRecRotate) != 0;
-    rec.crowd = (recs_.info & kRecCrowd) != 0;
-    rec.t[0] = recs_.t[0];
-    rec.t[1] = recs_.t[1];
-    rec.t[2] = recs_.t[2];
-    const int m = rec.m;
-    const int m0 = recs_.m0, n = recs_.info & kRecCount;
-    const int b = s & 1;
-    const bool same = (m == p_m) && p_acc;  // moved (and accepted) last step
-    // centre of m: the one this step's thread computed last step if m moved
-    // then, else the one loaded at the end of the previous step
-    float c0, c1, c2;
-    if (same && !p_rot) {
-      c0 = p_nc0;
-      c1 = p_nc1;
-      c2 = p_nc2;
-    } else {
-      const float4 c = A.mol_in_smem ? cent[m] : next_c;
-      c0 = c.x;
-      c1 = c.y;
-      c2 = c.z;
-    }
-    float nc0 = c0, nc1 = c1, nc2 = c2;
-    if (!rec.rotate) {
-      const float x0 = __fadd_rn(__fadd_rn(c0, rec.t[0]), box);
-      const float x1 = __fadd_rn(__fadd_rn(c1, rec.t[1]), box);
-      const float x2 = __fadd_rn(__fadd_rn(c2, rec.t[2]), box);
-      // c + t + L almost always lies in [0, 2L), where wrap_box subtracts L
-      // or nothing: one test for all three, selects instead of branches
-      const float L2 = 2.0f * box;  // exact
-      if (x0 >= 0.0f && x0 < L2 && x1 >= 0.0f && x1 < L2 && x2 >= 0.0f && x2 < L2) {
-        nc0 = x0 < box ? x0 : __fsub_rn(x0, box);
-        nc1 = x1 < box ? x1 : __fsub_rn(x1, box);
-        nc2 = x2 < box ? x2 : __fsub_rn(x2, box);
-      } else {
-        nc0 = wrap_box(x0, box);
-        nc1 = wrap_box(x1, box);
-        nc2 = wrap_box(x2, box);
-      }
-    }
-    // a one-bead rotation moves nothing (its bead sits at the centre): dE = 0
-    const bool skip = rec.rotate && n == 1;
-    float4 pold1, pnew1;  // one-bead molecule: old/new position in registers
-    if (n == 1) {
-      pold1 = same ? p_single : s_beads[m0];
-      pnew1 = make_float4(nc0, nc1, nc2, pold1.w);
-    } else {
-      // trial positions of the chain, built by the owners of its beads
-      QuatProducts qp{};
-      if (rec.rotate) qp = quat_products(recs_.q[0], recs_.q[1], recs_.q[2], recs_.q[3]);
-      int j = m0 + ((tid - m0) & tmask);
-      for (; j < m0 + n; j += nthr) {
-        const int k = j - m0;
-        const float4 rl = A.rel[bead_off + j];
-        // the bead's current position: this thread owns it and installed
-        // its last move itself
-        const float4 ol = s_beads[j];
-        float4 np;
-        if (rec.rotate) {
-          const float3 r2 = rotate_rel(qp, rl.x, rl.y, rl.z);
-          np = make_float4(__fadd_rn(r2.x, nc0), __fadd_rn(r2.y, nc1), __fadd_rn(r2.z, nc2), ol.w);
-          s_trel[b * A.lmax + k] = make_float4(r2.x, r2.y, r2.z, 0.0f);
-        } else {
-          np = make_float4(__fadd_rn(rl.x, nc0), __fadd_rn(rl.y, nc1), __fadd_rn(rl.z, nc2), ol.w);
-        }
-        float4* e = s_tpos + 2 * (b * A.lmax + k);
-        e[0] = make_float4(np.x, ol.x, np.y, ol.y);
-        e[1] = make_float4(np.z, ol.z, ol.w, __int_as_float(bead_type(ol.w) * kNT));
-      }
-      __syncthreads();  // trial positions and the previous chain update visible
-    }
-
-    // ---- dE over beads j outside the molecule (thread t owns j = t mod T).
-    // Beads are chains [0, ncb) then crowders [ncb, N); the moved molecule's
-    // own beads [m0, m0 + n) split the range in two. Residue-residue pairs of
-    // a chain move are the change of the chain-chain energy sample() adds.
-    double dacc = 0.0, dcc = 0.0;
-    if (!skip) {
-      const int x0 = m0, x1 = m0 + n;
-      float acc_c = 0.0f, acc_o = 0.0f;
-      if (n == 1) {
-        // one bead (a crowder or a one-residue chain), positions in registers
-        const int ta = bead_type(pold1.w);
-        const float4* trow = s_tab + ta * kNT;
-        if (rec.crowd) {
-          // a one-bead crowder: every pair is a crowder pair. One loop over
-          // the thread's j in increasing order (the order of the per-thread
-          // sum), two j per pass with both loads issued first, the moved
-          // bead itself (j = m0) left out of the sum
-          const bool one_ct = ctype >= 0;
-          const float4 Tc = trow[one_ct ? ctype : 0];
-          // the two beads of a pass as the two lanes of packed FP32, against
-          // the moved bead's new and old position (negated once per step)
-          const PackedBox PB1 = packed_box(box, invbox);
-          const float2 nnx = make_float2(-pnew1.x, -pnew1.x), nny = make_float2(-pnew1.y, -pnew1.y),
-                       nnz = make_float2(-pnew1.z, -pnew1.z);
-          const float2 nox = make_float2(-pold1.x, -pold1.x), noy = make_float2(-pold1.y, -pold1.y),
-                       noz = make_float2(-pold1.z, -pold1.z);
-          int j = gtid;
-          // folded minimum image where the system allows it (fold_mi)
-          auto pass1 = [&](auto fold) {
-            constexpr bool F = decltype(fold)::value;
-            for (; j + gstride < N; j += 2 * gstride) {
-              const int j2 = j + gstride;
-              const float4 pa = s_beads[j], pb = s_beads[j2];
-              const float4 Ta = (one_ct && j >= ncb) ? Tc : trow[bead_type(pa.w)];
-              const float4 Tb = (one_ct && j2 >= ncb) ? Tc : trow[bead_type(pb.w)];
-              const float2 xj = make_float2(pa.x, pb.x), yj = make_float2(pa.y, pb.y),
-                           zj = make_float2(pa.z, pb.z);
-              const float2 A2 = make_float2(Ta.x, Tb.x), C2 = make_float2(Ta.z, Tb.z);
-              const float2 en =
-                  crowd_energy2<R12, CUT>(pair_r2_2<F>(xj, yj, zj, nnx, nny, nnz, PB1), A2, C2);
-              const float2 eo =
-                  crowd_energy2<R12, CUT>(pair_r2_2<F>(xj, yj, zj, nox, noy, noz, PB1), A2, C2);
-              const float2 d = __fadd2_rn(en, make_float2(-eo.x, -eo.y));
-              if (j != m0) acc_o += d.x;
-              if (j2 != m0) acc_o += d.y;
-            }
-          };
-          if (S.fold_mi) pass1(std::true_type{}); else pass1(std::false_type{});
-          if (j < N && j != m0) {
-            const float4 pa = s_beads[j];
-            const float4 Ta = (one_ct && j >= ncb) ? Tc : trow[bead_type(pa.w)];
-            const float en = crowd_energy<R12, CUT>(pair_r2(pnew1, pa, box, invbox), Ta.x, Ta.z);
-            const float eo = crowd_energy<R12, CUT>(pair_r2(pold1, pa, box, invbox), Ta.x, Ta.z);
-            acc_o += en - eo;
-          }
-        } else {
-          // a one-residue chain: residue pairs with the chains' beads,
-          // crowder pairs with the rest
-          for (int part = 0; part < 2; ++part) {
-            const int lo = part ? x1 : 0, hi = part ? N : x0;
-            if (lo >= hi) continue;
-            const int cb = min(hi, ncb);
-            int j = lo + ((gtid - lo) & gmask);  // first j >= lo in this thread's class
-            for (; j < cb; j += gstride) {
-              const float4 pj = s_beads[j];
-              const float4 Tj = trow[bead_type(pj.w)];
-              const float en = pair_energy_r2(pair_r2(pnew1, pj, box, invbox), Tj, false, A.K);
-              const float eo = pair_energy_r2(pair_r2(pold1, pj, box, invbox), Tj, false, A.K);
-              acc_c += en - eo;
-            }
-            const float4 Tc = trow[ctype >= 0 ? ctype : 0];
-            for (; j < hi; j += gstride) {
-              const float4 pj = s_beads[j];
-              const float4 Tj = ctype >= 0 ? Tc : trow[bead_type(pj.w)];
-              const float en = crowd_energy<R12, CUT>(pair_r2(pnew1, pj, box, invbox), Tj.x, Tj.z);
-              const float eo = crowd_energy<R12, CUT>(pair_r2(pold1, pj, box, invbox), Tj.x, Tj.z);
-              acc_o += en - eo;
-            }
-          }
-        }
-      } else {
-        // a chain (or a multi-bead crowder): each thread takes its beads j and
-        // runs over the n moved beads k, the same k in every lane. Two j per
-        // pass where the class has them, so each k's positions and table row
-        // serve two beads; each j's sum over k is added on its own, in j order
-        const float4* tp = s_tpos + 2 * b * A.lmax;
-        for (int part = 0; part < 2; ++part) {
-          const int lo = part ? x1 : 0, hi = part ? N : x0;
-          if (lo >= hi) continue;
-          const int cb = min(hi, ncb);
-          int j = lo + ((gtid - lo) & gmask);
-          if (!rec.crowd) {
-            // residue pairs: the new and the old evaluation of a pair as the
-            // two lanes of packed FP32
-            const PackedBox PB = packed_box(box, invbox);
-            auto pass2 = [&](auto fold) {
-              constexpr bool F = decltype(fold)::value;
-              for (; j + gstride < cb; j += 2 * gstride) {
-                const float4 pa = s_beads[j], pb = s_beads[j + gstride];
-                const int ta = bead_type(pa.w), tb = bead_type(pb.w);
-                const float2 nax = make_float2(-pa.x, -pa.x), nay = make_float2(-pa.y, -pa.y),
-                             naz = make_float2(-pa.z, -pa.z);
-                const float2 nbx = make_float2(-pb.x, -pb.x), nby = make_float2(-pb.y, -pb.y),
-                             nbz = make_float2(-pb.z, -pb.z);
-                float a = 0.0f, c = 0.0f;
-#pragma unroll 2
-                for (int k = 0; k < n; ++k) {
-                  const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-                  const float2 kx = make_float2(P.x, P.y), ky = make_float2(P.z, P.w),
-                               kz = make_float2(Q.x, Q.y);
-                  const float4* row = s_tab + __float_as_int(Q.w);
-                  const float4 Ta = row[ta], Tb = row[tb];
-                  const float2 ea =
-                      kh_energy2(pair_r2_2<F>(kx, ky, kz, nax, nay, naz, PB), Ta, A.K.c_xi);
-                  const float2 eb =
-                      kh_energy2(pair_r2_2<F>(kx, ky, kz, nbx, nby, nbz, PB), Tb, A.K.c_xi);
-                  a += ea.x - ea.y;
-                  c += eb.x - eb.y;
-                }
-                acc_c += a;
-                acc_c += c;
-              }
-            };
-            if (S.fold_mi) pass2(std::true_type{}); else pass2(std::false_type{});
-          }
-          for (; j < cb; j += gstride) {
-            const float4 pj = s_beads[j];
-            const int tb = bead_type(pj.w);
-            float a = 0.0f;
-            if (!rec.crowd) {
-              for (int k = 0; k < n; ++k) {
-                const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-                const float4 pn = make_float4(P.x, P.z, Q.x, 0.0f), po = make_float4(P.y, P.w, Q.y, 0.0f);
-                const float4 T = s_tab[__float_as_int(Q.w) + tb];
-                const float en = pair_energy_r2(pair_r2(pn, pj, box, invbox), T, false, A.K);
-                const float eo = pair_energy_r2(pair_r2(po, pj, box, invbox), T, false, A.K);
-                a += en - eo;
-              }
-              acc_c += a;
-            } else {
-              for (int k = 0; k < n; ++k) {
-                const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-                const float4 pn = make_float4(P.x, P.z, Q.x, 0.0f), po = make_float4(P.y, P.w, Q.y, 0.0f);
-                const float4 T = s_tab[__float_as_int(Q.w) + tb];
-                const float en = crowd_energy<R12, CUT>(pair_r2(pn, pj, box, invbox), T.x, T.z);
-                const float eo = crowd_energy<R12, CUT>(pair_r2(po, pj, box, invbox), T.x, T.z);
-                a += en - eo;
-              }
-              acc_o += a;
-            }
-          }
-          const bool one_ct = ctype >= 0;
-          const PackedBox PBc = packed_box(box, invbox);
-          auto pass3 = [&](auto fold) {
-            constexpr bool F = decltype(fold)::value;
-            for (; j + gstride < hi; j += 2 * gstride) {
-              const float4 pa = s_beads[j], pb = s_beads[j + gstride];
-              const int ta = bead_type(pa.w), tb = bead_type(pb.w);
-              const float2 nax = make_float2(-pa.x, -pa.x), nay = make_float2(-pa.y, -pa.y),
-                           naz = make_float2(-pa.z, -pa.z);
-              const float2 nbx = make_float2(-pb.x, -pb.x), nby = make_float2(-pb.y, -pb.y),
-                           nbz = make_float2(-pb.z, -pb.z);
-              float a = 0.0f, c = 0.0f;
-#pragma unroll 2
-              for (int k = 0; k < n; ++k) {
-                const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-                const float2 kx = make_float2(P.x, P.y), ky = make_float2(P.z, P.w),
-                             kz = make_float2(Q.x, Q.y);
-                const float4* row = s_tab + __float_as_int(Q.w);
-                const float4 Ta = row[ta];
-                const float4 Tb = one_ct ? Ta : row[tb];  // one crowder species: ta == tb
-                const float2 ea = crowd_energy2<R12, CUT>(pair_r2_2<F>(kx, ky, kz, nax, nay, naz, PBc),
-                                                          make_float2(Ta.x, Ta.x),
-                                                          make_float2(Ta.z, Ta.z));
-                const float2 eb = crowd_energy2<R12, CUT>(pair_r2_2<F>(kx, ky, kz, nbx, nby, nbz, PBc),
-                                                          make_float2(Tb.x, Tb.x),
-                                                          make_float2(Tb.z, Tb.z));
-                a += ea.x - ea.y;
-                c += eb.x - eb.y;
-              }
-              acc_o += a;
-              acc_o += c;
-            }
-          };
-          if (S.fold_mi) pass3(std::true_type{}); else pass3(std::false_type{});
-          for (; j < hi; j += gstride) {
-            const float4 pj = s_beads[j];
-            const int tb = bead_type(pj.w);
-            float a = 0.0f;
-            for (int k = 0; k < n; ++k) {
-              const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-              const float4 pn = make_float4(P.x, P.z, Q.x, 0.0f), po = make_float4(P.y, P.w, Q.y, 0.0f);
-              const float4 T = s_tab[__float_as_int(Q.w) + tb];
-              const float en = crowd_energy<R12, CUT>(pair_r2(pn, pj, box, invbox), T.x, T.z);
-              const float eo = crowd_energy<R12, CUT>(pair_r2(po, pj, box, invbox), T.x, T.z);
-              a += en - eo;
-            }
-            acc_o += a;
-          }
-        }
-      }
-      dcc = (double)acc_c;
-      dacc = (double)acc_o;
-    }
-    dacc = warp_sum(dacc);
-    if (!rec.crowd) dcc = warp_sum(dcc);
-    if (lane == 0) {
-      if (!CLUSTER) {
-        s_red[b * 64 + warp] = dacc;
-        s_red[b * 64 + 32 + warp] = dcc;
-      } else {
-        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-        for (int r = 0; r < csize; ++r) {
-          double* dst = cl.map_shared_rank(s_red, r) + (b * csize + crank) * 64;
-          dst[warp] = dacc;
-          dst[32 + warp] = dcc;
-        }
-      }
-    }
-    if ((s & 31) == 31) cp_async_wait_all();  // next ring half has landed
-    // R: partial sums (and the prefetched records) visible
-    if (!CLUSTER)
-      __syncthreads();
-    else
-      cooperative_groups::this_cluster().sync();
-
-    // ---- every thread: the same FP64 sums (a fixed pairwise tree over the
-    // warps' partials) and the same Metropolis decision
-    if (s + 1 < n_steps && A.mol_in_smem == 0) {
-      next_c = cent[s_ring[(s + 1) & (kRing - 1)].m];
-    }
-    double dE = tree_sum8(s_red + b * csize * 64);
-    double dE_cc = 0.0;
-    if (!rec.crowd) dE_cc = tree_sum8(s_red + b * csize * 64 + 32);
-    for (int r = 1; r < csize; ++r) {  // the other CTAs' sums, in rank order
-      dE += tree_sum8(s_red + (b * csize + r) * 64);
-      if (!rec.crowd) dE_cc += tree_sum8(s_red + (b * csize + r) * 64 + 32);
-    }
-    if (!rec.crowd) dE += dE_cc;
-    const int acc = dE < 0.0 ? 1 : (dE < recs_.thr ? 2 : 0);
-    if (acc) {
-      energy += dE;
-      ecc += dE_cc;
-      if (n == 1) {
-        if (tid == (m0 & tmask)) s_beads[m0] = pnew1;
-        p_single = pnew1;
-      } else {
-        // the owners install the chain (and its relative positions)
-        int j = m0 + ((tid - m0) & tmask);
-        for (; j < m0 + n; j += nthr) {
-          const float4* e = s_tpos + 2 * (b * A.lmax + (j - m0));
-          const float4 P = e[0], Q = e[1];
-          s_beads[j] = make_float4(P.x, P.z, Q.x, Q.z);
-          if (rec.rotate) A.rel[bead_off + j] = s_trel[b * A.lmax + (j - m0)];
-        }
-      }
-      if (tid == 0 && rec.rotate && crank == 0) {
-        double* qd = A.quat + 4 * (size_t)(mol_off + m);
-        double out[4];
-        quat_mul(recs_.q[0], recs_.q[1], recs_.q[2], recs_.q[3], qd[0], qd[1], qd[2], qd[3], out);
-        qd[0] = out[0];
-        qd[1] = out[1];
-        qd[2] = out[2];
-        qd[3] = out[3];
-      }
-      if (tid == 0 && !rec.rotate) cent[m] = make_float4(nc0, nc1, nc2, 0.0f);
-    }
-    // counters: every thread keeps them (no branch on the thread index);
-    // thread 0 of rank 0 writes them out
-    n_neg += acc == 1;
-    n_boltz += acc == 2;
-    n_rej += acc == 0;
-    if (!skip) {
-      // two evaluations (old and new position) per pair
-      const unsigned nn2 = 2u * (unsigned)n;
-      if (rec.crowd) {
-        ev_crowd += (unsigned long long)nn2 * (unsigned)(N - n);
-      } else {
-        ev_kh += (unsigned long long)nn2 * (unsigned)(S.n_chain_beads - n);
-        ev_crowd += (unsigned long long)nn2 * (unsigned)(N - S.n_chain_beads);
-      }
-    }
-    // ---- Replica::sample at the end of every sampling chunk (main.cpp:975-989):
-    // bound if potential (+ chain-chain energy when crowders exist) < threshold
-    if (to_sample > 0 && --to_sample == 0) {
-      to_sample = A.sample_every;
-      const uint32_t label = step0 + (uint32_t)(s + 1 - A.sample_every);
-      if (label >= A.sample_after) {
-        const double enc = (ncb < N) ? energy + ecc : energy;
-        const bool bound = enc < A.bound_thr;
-        ++n_samp;  // every thread; thread 0 of rank 0 writes them out
-        n_bnd += bound ? 1 : 0;
-        if (bound && A.sample_out && crank == 0) {
-          __syncthreads();  // this step's centre / rotation writes visible
-          if (tid == 0) {
-            const unsigned r = atomicAdd(&A.sample_cursor[0], 1u);
-            const unsigned p0 = atomicAdd(&A.sample_cursor[1], (unsigned)M);
-            if (r < A.sample_cap && (unsigned long long)p0 + M <= A.pose_cap) {
-              SampleHeader hd;
-              hd.inst = inst;
-              hd.label = label;
-              hd.e_nc = enc;
-              hd.e = energy;
-              hd.temperature = A.ladder[S.inst0 + A.temp_idx[inst]];
-              hd.n_mol = M;
-              hd.pose_offset = p0;
-              hd.pad = 0;
-              A.sample_out[r] = hd;
-              s_pose_slot = p0;
-            } else {
-              atomicAdd(&A.sample_cursor[2], 1u);
-              s_pose_slot = -1;
-            }
-          }
-          __syncthreads();
-          const long long p0 = s_pose_slot;
-          if (p0 >= 0) {
-            for (int i = tid; i < M; i += nthr) {
-              const double* qd = A.quat + 4 * (size_t)(mol_off + i);
-              const float4 c = cent[i];
-              SamplePose ps;
-              ps.q[0] = qd[0];
-              ps.q[1] = qd[1];
-              ps.q[2] = qd[2];
-              ps.q[3] = qd[3];
-              ps.c[0] = c.x;
-              ps.c[1] = c.y;
-              ps.c[2] = c.z;
-              ps.pad = 0.0f;
-              A.pose_out[p0 + i] = ps;
-            }
-          }
-          __syncthreads();  // poses read before the next step moves anything
-        }
-      }
-    }
-    p_m = m;
-    p_acc = acc != 0;
-    p_rot = rec.rotate;
-    p_n = n;
-    p_b = b;
-    p_nc0 = nc0;
-    p_nc1 = nc1;
-    p_nc2 = nc2;
-  }
-  (void)p_n;
-  __syncthreads();
-
-  // ---- epilogue: write the instance back (every CTA of a cluster holds the
-  // same state; rank 0 writes it)
-  if (crank == 0) {
-  if (!GB)
-    for (int i = tid; i < N; i += nthr) A.pos[bead_off + i] = s_beads[i];
-  if (A.mol_in_smem)
-    for (int i = tid; i < M; i += nthr) A.centre[mol_off + i] = s_cent[i];
-  }
-  if (tid == 0 && crank == 0) {
-    A.energy[inst] = energy;
-    A.ecc[inst] = ecc;
-    A.n_samples[inst] += n_samp;
-    A.n_bound[inst] += n_bnd;
-    A.acc_neg[inst] += n_neg;
-    A.acc_boltz[inst] += n_boltz;
-    A.rej[inst] += n_rej;
-    A.evals_kh[inst] += ev_kh;
-    A.evals_crowd[inst] += ev_crowd;
-  }
-  __syncthreads();  // shared memory is reused by the next instance
-  }  // instance loop
-  // no CTA leaves while another may still write into its shared memory
-  if (CLUSTER) cooperative_groups::this_cluster().sync();
 }
 
 // ------------------------------------------------------------------ state staging
@@ -1926,9 +1188,9 @@ struct remc_handle {
   int sweep_csize = 1; // CTAs per replica (thread-block cluster size)
   int sweep_cluster_slots = 0;  // clusters of that size the GPU holds at once
   int beads_in_smem = 1; // beads resident in shared memory (else updated in place in global)
-  float4* d_trial_scratch = nullptr;  // sweep trial buffers, 6 lmax per (instance, CTA rank)
+  float4* d_sweep_scratch = nullptr;  // what a sweep CTA does not hold in shared memory
   float* d_fold_part = nullptr;       // per instance: the fold test's partial extents [8]
-  size_t trial_scratch_cap = 0;       // float4 entries
+  size_t sweep_scratch_cap = 0;       // float4 entries
   int max_dyn_smem = 0;
   int config_gen = 0;  // bumped when the sweep schedule changes
   TileItem* d_items_by_cost = nullptr;  // the items by decreasing cost (work-queue order)
@@ -1965,7 +1227,11 @@ struct remc_handle {
   double* d_stage_q = nullptr; // quaternions [4m]
   unsigned long long* d_bad = nullptr;  // first invalid bead / one-bead offset / molecule
   int* d_err = nullptr;        // set by a kernel whose bounded wait gave up
-  int sweep_threads = 128;
+  int sweep_threads = 128;  // virtual threads per CTA (the schedule's threads per replica)
+  int sweep_block = 256;    // threads per CTA
+  SweepShape sweep_shape{};
+  bool all_fold = false;    // every system's fold flag is set (the state uploaded last)
+  int nrel = 0;             // beads up to the last one of a molecule of several
   int num_sms = 148;
   // graph
   cudaGraphExec_t graph_exec = nullptr;
@@ -2001,7 +1267,7 @@ void free_all(remc_handle* h) {
                   h->d_ctrl,     h->d_items_by_cost, h->d_energy_queue,
                   h->d_item_off,   h->d_scratch,    h->d_newpos,
                   h->d_dE,       h->d_bead_info, h->d_stage,      h->d_stage_q,    h->d_bad,
-                  h->d_err,      h->d_trial_scratch, h->d_fold_part};
+                  h->d_err,      h->d_sweep_scratch, h->d_fold_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
@@ -2101,41 +1367,91 @@ int ensure_recs(remc_handle* h, size_t steps) {
   return REMC_OK;
 }
 
-// The sweep kernel compiled for the handle's crowder model, single CTAs or
-// clusters of CTAs per replica, beads in shared or in global memory.
-using SweepFn = void (*)(SweepArgs);
-template <bool CLUSTER, bool GB>
-SweepFn sweep_fn_model(const remc_params& p) {
-  const bool cut = p.crowder_cutoff > 0.0f;
-  if (p.crowder_mode)
-    return cut ? sweep_kernel<true, true, CLUSTER, GB> : sweep_kernel<true, false, CLUSTER, GB>;
-  return cut ? sweep_kernel<false, true, CLUSTER, GB> : sweep_kernel<false, false, CLUSTER, GB>;
-}
-SweepFn sweep_fn(const remc_params& p, bool cluster, bool global_beads) {
-  if (global_beads)
-    return cluster ? sweep_fn_model<true, true>(p) : sweep_fn_model<false, true>(p);
-  return cluster ? sweep_fn_model<true, false>(p) : sweep_fn_model<false, false>(p);
+SweepFn sweep_fn(const remc_handle* h, bool cluster, bool global_beads) {
+  const bool cut = h->params.crowder_cutoff > 0.0f, fold = h->all_fold;
+  return h->params.crowder_mode ? sweep_fn_wall(cut, fold, cluster, global_beads)
+                                : sweep_fn_reference(cut, fold, cluster, global_beads);
 }
 
-// Set the sweep schedule: threads per replica, where molecule data lives,
-// CTAs per replica, and whether the beads are resident in shared memory.
+// Shared-memory shape of a sweep launch, without the parts it can do without.
+SweepShape base_shape(const remc_handle* h, int threads, int mol_in_smem, int csize,
+                      int beads_in_smem) {
+  SweepShape p{};
+  p.nmax = h->nmax;
+  p.mmax = h->mmax;
+  p.lmax = h->lmax;
+  p.nrel = h->nrel;
+  p.csize = csize;
+  p.vthreads = threads;
+  p.mol_in_smem = mol_in_smem;
+  p.beads_in_smem = beads_in_smem;
+  return p;
+}
+
+// Scratch entries per (instance, CTA rank): trial positions and relative
+// positions, then a chain step's sums per bead.
+size_t scratch_stride(const SweepShape& p) {
+  return 3 * (size_t)p.lmax + ((size_t)local_beads(p) + 3) / 4;
+}
+int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
+  if (p.aj_in_smem && p.beads_in_smem) return REMC_OK;
+  const size_t need = (size_t)h->n_inst * p.csize * scratch_stride(p);
+  if (need <= h->sweep_scratch_cap) return REMC_OK;
+  float4* q = nullptr;
+  if (dev_alloc(&q, need)) return REMC_ERR_NOMEM;
+  if (h->d_sweep_scratch) {
+    cudaStreamSynchronize(h->stream);
+    cudaFree(h->d_sweep_scratch);
+  }
+  h->d_sweep_scratch = q;
+  h->sweep_scratch_cap = need;
+  h->config_gen++;  // a captured graph holds the old pointer
+  return REMC_OK;
+}
+
+// Set the sweep schedule: virtual threads per CTA (they fix the order of the
+// sums, see remc_sweep.cuh), where molecule data lives, CTAs per replica, and
+// whether the beads are resident in shared memory.
 int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int beads_in_smem) {
   if (threads < 32 || threads > 256 || (threads & (threads - 1)) != 0)
     return set_error(REMC_ERR_INVALID, "threads per replica must be 32, 64, 128 or 256");
   if (csize != 1 && csize != 2 && csize != 4 && csize != 8)
     return set_error(REMC_ERR_INVALID, "cluster size must be 1, 2, 4 or 8");
-  const size_t smem =
-      SweepSmem::make(h->nmax, h->mmax, h->lmax, mol_in_smem, csize, beads_in_smem).total;
-  if (smem > (size_t)h->max_dyn_smem)
+  SweepShape shape = base_shape(h, threads, mol_in_smem, csize, beads_in_smem);
+  const size_t least = SweepSmem::make(shape).total;
+  if (least > (size_t)h->max_dyn_smem)
     return set_error(REMC_ERR_INVALID,
-                     "largest system needs %zu bytes of shared memory, device allows %d", smem,
+                     "largest system needs %zu bytes of shared memory, device allows %d", least,
                      h->max_dyn_smem);
-  const SweepFn fn = sweep_fn(h->params, csize > 1, !beads_in_smem);
+  const SweepFn fn = sweep_fn(h, csize > 1, !beads_in_smem);
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+  // two warps per virtual warp: a group of 8 steps then has whole warps (128
+  // virtual threads) or pairs of warps (256) for every step
+  const int block = std::min(kSweepThreads, std::max(256, 2 * threads));
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, least);
   if (e != cudaSuccess || per_sm < 1)
     return set_error(REMC_ERR_CUDA, "sweep kernel does not fit on an SM: %s",
                      cudaGetErrorString(e));
+  // what fits beside it without taking CTAs off the SM
+  auto fits = [&](const SweepShape& p) {
+    const size_t smem = SweepSmem::make(p).total;
+    int n = 0;
+    return smem <= (size_t)h->max_dyn_smem &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) == cudaSuccess &&
+           n >= per_sm;
+  };
+  auto add = [&](int SweepShape::*what, int value) {
+    SweepShape p = shape;
+    p.*what = value;
+    if (!fits(p)) return false;
+    shape = p;
+    return true;
+  };
+  add(&SweepShape::aj_in_smem, 1);
+  for (int cap = 4096; cap >= 1024 && !add(&SweepShape::term_cap, cap); cap /= 2) {
+  }
+  if (beads_in_smem) add(&SweepShape::rel_in_smem, 1);
+  const size_t smem = SweepSmem::make(shape).total;
   if (csize > 1) {
     // the cluster must be schedulable: csize CTAs of this size in one GPC
     cudaLaunchConfig_t cfg = {};
@@ -2145,7 +1461,7 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(csize);
-    cfg.blockDim = dim3(threads);
+    cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -2156,23 +1472,10 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
                        cudaGetErrorString(e));
     h->sweep_cluster_slots = clusters;
   }
-  {
-    // trial buffers of every (instance, CTA rank): 6 lmax float4 each (the
-    // trial relative positions, and the trial positions when the beads stay
-    // in global memory)
-    const size_t need = (size_t)h->n_inst * csize * 6 * (size_t)h->lmax;
-    if (need > h->trial_scratch_cap) {
-      float4* p = nullptr;
-      if (dev_alloc(&p, need)) return REMC_ERR_NOMEM;
-      if (h->d_trial_scratch) {
-        cudaStreamSynchronize(h->stream);
-        cudaFree(h->d_trial_scratch);
-      }
-      h->d_trial_scratch = p;
-      h->trial_scratch_cap = need;
-    }
-  }
+  if (ensure_sweep_scratch(h, shape)) return REMC_ERR_NOMEM;
+  h->sweep_shape = shape;
   h->sweep_threads = threads;
+  h->sweep_block = block;
   h->mol_in_smem = mol_in_smem;
   h->sweep_csize = csize;
   h->beads_in_smem = beads_in_smem;
@@ -2227,7 +1530,6 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   if (csize > 1) persistent = false;
   A.queue = persistent ? h->d_queue : nullptr;
   A.n_list = n_blocks;
-  A.csize = csize;
   if (persistent) {
     REMC_CUDA_TRY(cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream));
     n_blocks = std::min(n_blocks, h->sweep_grid);
@@ -2236,7 +1538,6 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   A.rel = h->d_rel;
   A.centre = h->d_centre;
   A.quat = h->d_quat;
-  A.mol_start = h->d_mol_start;
   A.tab = h->d_tab;
   A.recs = h->d_recs;
   A.energy = h->d_energy;
@@ -2263,17 +1564,16 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   A.rec_stride = (int)h->recs_cap;
   A.rec_offset = rec_offset;
   A.n_steps = n_steps;
-  A.nmax = h->nmax;
-  A.mmax = h->mmax;
-  A.mol_in_smem = h->mol_in_smem;
-  A.lmax = h->lmax;
-  A.trial_scratch = h->d_trial_scratch;
+  A.shape = csize == h->sweep_csize
+                ? h->sweep_shape
+                : base_shape(h, h->sweep_threads, h->mol_in_smem, csize, h->beads_in_smem);
+  A.scratch = h->d_sweep_scratch;
+  A.scratch_stride = (long long)scratch_stride(A.shape);
   A.K = consts_of(h);
   const bool gb = !h->beads_in_smem;
-  const size_t smem =
-      SweepSmem::make(h->nmax, h->mmax, h->lmax, h->mol_in_smem, csize, h->beads_in_smem).total;
+  const size_t smem = SweepSmem::make(A.shape).total;
   if (csize == 1) {
-    sweep_fn(h->params, false, gb)<<<n_blocks, h->sweep_threads, smem, h->stream>>>(A);
+    sweep_fn(h, false, gb)<<<n_blocks, h->sweep_block, smem, h->stream>>>(A);
   } else {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -2282,12 +1582,12 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(csize * n_blocks);
-    cfg.blockDim = dim3(h->sweep_threads);
+    cfg.blockDim = dim3(h->sweep_block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = h->stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    REMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, sweep_fn(h->params, true, gb), A));
+    REMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, sweep_fn(h, true, gb), A));
   }
   REMC_CUDA_TRY(cudaGetLastError());
   return REMC_OK;
@@ -2444,6 +1744,8 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
     h->nmax = std::max(h->nmax, d.n_beads);
     h->mmax = std::max(h->mmax, d.n_mol);
     h->lmax = std::max(h->lmax, lmax);
+    for (int m = 0; m < d.n_mol; ++m)
+      if (d.mol_start[m + 1] - d.mol_start[m] > 1) h->nrel = std::max(h->nrel, d.mol_start[m + 1]);
   }
   if (bead_cursor >= (size_t)1 << 31) {
     delete h;
@@ -2461,15 +1763,11 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
-  const SweepFn kSweeps[16] = {
-      sweep_kernel<false, false, false, false>, sweep_kernel<false, true, false, false>,
-      sweep_kernel<true, false, false, false>,  sweep_kernel<true, true, false, false>,
-      sweep_kernel<false, false, true, false>,  sweep_kernel<false, true, true, false>,
-      sweep_kernel<true, false, true, false>,   sweep_kernel<true, true, true, false>,
-      sweep_kernel<false, false, false, true>,  sweep_kernel<false, true, false, true>,
-      sweep_kernel<true, false, false, true>,   sweep_kernel<true, true, false, true>,
-      sweep_kernel<false, false, true, true>,   sweep_kernel<false, true, true, true>,
-      sweep_kernel<true, false, true, true>,    sweep_kernel<true, true, true, true>};
+  SweepFn kSweeps[32];
+  for (int k = 0; k < 16; ++k) {
+    kSweeps[k] = sweep_fn_wall(k & 1, k & 2, k & 4, k & 8);
+    kSweeps[16 + k] = sweep_fn_reference(k & 1, k & 2, k & 4, k & 8);
+  }
   int static_smem = 0;
   for (SweepFn f : kSweeps) {
     cudaFuncAttributes fattr;
@@ -2494,7 +1792,10 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   // beads left in global memory for systems too large for shared memory
   {
     const int threads = h->nmax <= 2048 ? 128 : 256;
-    int rc0 = configure_sweep(h, threads, 1, 1, 1);
+    // centres in shared memory only where clusters of any size keep them too
+    // (a cluster's CTAs exchange more sums)
+    const bool centres = SweepSmem::make(base_shape(h, threads, 1, 8, 1)).total <= (size_t)max_dyn;
+    int rc0 = centres ? configure_sweep(h, threads, 1, 1, 1) : REMC_ERR_INVALID;
     if (rc0) rc0 = configure_sweep(h, threads, 0, 1, 1);
     if (rc0) rc0 = configure_sweep(h, threads, 0, 1, 0);
     if (rc0) {
@@ -2745,6 +2046,15 @@ int remc_upload_state(remc_handle* h, const float* pos, const float* rel, const 
   REMC_CUDA_TRY(cudaGetLastError());
   REMC_CUDA_TRY(cudaMemcpyAsync(h->d_quat, h->d_stage_q, sizeof(double) * 4 * nm,
                                 cudaMemcpyDeviceToDevice, h->stream));
+  // the sweep folds the minimum image where every system allows it
+  std::vector<SysDev> sd(h->n_sys);
+  REMC_CUDA_TRY(cudaMemcpyAsync(sd.data(), h->d_sys, sizeof(SysDev) * h->n_sys,
+                                cudaMemcpyDeviceToHost, h->stream));
+  REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  bool fold = true;
+  for (const SysDev& S : sd) fold = fold && S.fold_mi;
+  if (fold != h->all_fold) h->config_gen++;  // a captured graph holds the other kernel
+  h->all_fold = fold;
   h->state_set = true;
   return REMC_OK;
 }
@@ -2859,6 +2169,10 @@ int remc_sweep_plain(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0)
   int rc = check_ready(h);
   if (rc) return rc;
   if (n_steps < 0) return set_error(REMC_ERR_INVALID, "n_steps < 0");
+  if (h->sweep_csize > 1) {  // single CTAs all the same
+    rc = ensure_sweep_scratch(h, base_shape(h, h->sweep_threads, h->mol_in_smem, 1, h->beads_in_smem));
+    if (rc) return rc;
+  }
   const size_t chunk_max = max_chunk_steps(h);
   for (int done = 0; done < n_steps;) {
     const int chunk = (int)std::min((size_t)(n_steps - done), chunk_max);
