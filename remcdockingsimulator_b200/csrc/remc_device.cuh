@@ -276,6 +276,9 @@ __device__ __forceinline__ float2 crowd_change2(float2 rn, float2 ro, float2 A, 
 // entry T (the moved bead's new and old position against one bead j), in
 // packed FP32: pair_energy_r2's operations for a residue pair, with the last
 // product unrounded in the sum.
+// DH = false: T.w is zero (one of the residues is uncharged), the Debye-Hueckel
+// term drops out (0 * rinv keeps the NaN of coincident beads).
+template <bool DH = true>
 __device__ __forceinline__ float2 kh_energy2(float2 r2, float4 T, float c_xi) {
   const float2 rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
   const float2 rinv2 = __fmul2_rn(rinv, rinv);
@@ -287,6 +290,7 @@ __device__ __forceinline__ float2 kh_energy2(float2 r2, float4 T, float c_xi) {
       __ffma2_rn(make_float2(0.5f, 0.5f), make_float2(T.x, T.x), make_float2(-lj.x, -lj.y));
   lj.x = (r2.x < T.z) ? ljr.x : lj.x;  // repulsive branch: 2 eps' - LJ
   lj.y = (r2.y < T.z) ? ljr.y : lj.y;
+  if constexpr (!DH) return __ffma2_rn(make_float2(T.w, T.w), rinv, lj);
   const float2 r = __fmul2_rn(r2, rinv);
   const float2 arg = __fmul2_rn(r, make_float2(c_xi, c_xi));
   const float2 ex = make_float2(fast_ex2(arg.x), fast_ex2(arg.y));

@@ -1232,6 +1232,8 @@ struct remc_handle {
   SweepShape sweep_shape{};
   bool all_fold = false;    // every system's fold flag is set (the state uploaded last)
   int nrel = 0;             // beads up to the last one of a molecule of several
+  bool any_crowders = false;
+  double chain_step_pairs = 0.0;  // pairs of a step of a molecule of several beads, on average
   int num_sms = 148;
   // graph
   cudaGraphExec_t graph_exec = nullptr;
@@ -1381,7 +1383,7 @@ SweepShape base_shape(const remc_handle* h, int threads, int mol_in_smem, int cs
   p.mmax = h->mmax;
   p.lmax = h->lmax;
   p.nrel = h->nrel;
-  p.csize = csize;
+  p.csize = p.vsize = csize;
   p.vthreads = threads;
   p.mol_in_smem = mol_in_smem;
   p.beads_in_smem = beads_in_smem;
@@ -1391,7 +1393,7 @@ SweepShape base_shape(const remc_handle* h, int threads, int mol_in_smem, int cs
 // Scratch entries per (instance, CTA rank): trial positions and relative
 // positions, then a chain step's sums per bead.
 size_t scratch_stride(const SweepShape& p) {
-  return 3 * (size_t)p.lmax + ((size_t)local_beads(p) + 3) / 4;
+  return 3 * (size_t)p.lmax + ((size_t)held_sums(p) + 3) / 4;
 }
 int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
   if (p.aj_in_smem && p.beads_in_smem) return REMC_OK;
@@ -1409,6 +1411,60 @@ int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
   return REMC_OK;
 }
 
+// A cluster barrier with its remote stores costs some 1,500 cycles a pass, the
+// pairs of a chain step some 0.6 cycles each on one SM: a quarter of them per
+// CTA saves more from about 4,000 pairs on. Two chains of 76 and 24 residues
+// (1,824 pairs): 3.62 ms per 1000 steps spread, 3.15 not; 129 + 57 + 201
+// residues and 233 crowders (63,000): 0.80 ms spread, 1.17 not.
+constexpr double kSpreadPairs = 4096.0;
+
+// Add to a shape what fits in shared memory beside it without taking CTAs off
+// the SM, and find how many CTAs an SM, and clusters the GPU, hold.
+int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* clusters) {
+  const SweepFn fn = sweep_fn(h, shape.csize > 1, !shape.beads_in_smem);
+  auto resident = [&](const SweepShape& p) {
+    const size_t smem = SweepSmem::make(p).total;
+    int n = 0;
+    if (smem > (size_t)h->max_dyn_smem ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
+      return 0;
+    return n;
+  };
+  *per_sm = resident(shape);
+  if (*per_sm < 1) return set_error(REMC_ERR_CUDA, "sweep kernel does not fit on an SM");
+  auto add = [&](int SweepShape::*what, int value) {
+    SweepShape p = shape;
+    p.*what = value;
+    if (resident(p) < *per_sm) return false;
+    shape = p;
+    return true;
+  };
+  add(&SweepShape::aj_in_smem, 1);
+  for (int cap = 4096; cap >= 1024 && !add(&SweepShape::term_cap, cap); cap /= 2) {
+  }
+  if (shape.beads_in_smem) add(&SweepShape::rel_in_smem, 1);
+  *clusters = 0;
+  if (shape.csize > 1) {
+    // the cluster must be schedulable: csize CTAs of this size in one GPC
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = shape.csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(shape.csize);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = SweepSmem::make(shape).total;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(clusters, fn, &cfg);
+    if (e != cudaSuccess || *clusters < 1)
+      return set_error(REMC_ERR_INVALID, "a cluster of %d sweep CTAs does not fit: %s", shape.csize,
+                       cudaGetErrorString(e));
+  }
+  return REMC_OK;
+}
+
 // Set the sweep schedule: virtual threads per CTA (they fix the order of the
 // sums, see remc_sweep.cuh), where molecule data lives, CTAs per replica, and
 // whether the beads are resident in shared memory.
@@ -1423,55 +1479,32 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
     return set_error(REMC_ERR_INVALID,
                      "largest system needs %zu bytes of shared memory, device allows %d", least,
                      h->max_dyn_smem);
-  const SweepFn fn = sweep_fn(h, csize > 1, !beads_in_smem);
-  int per_sm = 0;
-  // two warps per virtual warp: a group of 8 steps then has whole warps (128
-  // virtual threads) or pairs of warps (256) for every step
-  const int block = std::min(kSweepThreads, std::max(256, 2 * threads));
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, least);
-  if (e != cudaSuccess || per_sm < 1)
-    return set_error(REMC_ERR_CUDA, "sweep kernel does not fit on an SM: %s",
-                     cudaGetErrorString(e));
-  // what fits beside it without taking CTAs off the SM
-  auto fits = [&](const SweepShape& p) {
-    const size_t smem = SweepSmem::make(p).total;
-    int n = 0;
-    return smem <= (size_t)h->max_dyn_smem &&
-           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) == cudaSuccess &&
-           n >= per_sm;
-  };
-  auto add = [&](int SweepShape::*what, int value) {
-    SweepShape p = shape;
-    p.*what = value;
-    if (!fits(p)) return false;
-    shape = p;
-    return true;
-  };
-  add(&SweepShape::aj_in_smem, 1);
-  for (int cap = 4096; cap >= 1024 && !add(&SweepShape::term_cap, cap); cap /= 2) {
+  // Two warps per virtual warp: a group of 8 steps then has whole warps (128
+  // virtual threads) or pairs of warps (256) for every step. Systems without
+  // crowders have chain steps only, which all threads share: 512
+  const int block = h->any_crowders ? std::min(kSweepThreads, std::max(256, 2 * threads)) : kSweepThreads;
+  int per_sm = 0, clusters = 0;
+  const int rc = fit_sweep(h, shape, block, &per_sm, &clusters);
+  if (rc) return rc;
+  // Replicas fewer than the SMs: a replica of one virtual CTA spreads over a
+  // cluster of up to four, each on its own SM, where its chain steps are long
+  // enough (kSpreadPairs) for the cluster barrier they then take.
+  if (csize == 1 && beads_in_smem && h->chain_step_pairs >= kSpreadPairs) {
+    for (int c = 4; c > 1; c /= 2) {
+      if ((long long)h->n_inst * c > h->num_sms) continue;
+      SweepShape wide = base_shape(h, threads, mol_in_smem, c, beads_in_smem);
+      wide.vsize = 1;
+      wide.aj_in_smem = 1;
+      int n = 0, k = 0;
+      if (SweepSmem::make(wide).total > (size_t)h->max_dyn_smem || fit_sweep(h, wide, block, &n, &k))
+        continue;
+      shape = wide;
+      per_sm = n;
+      clusters = k;
+      break;
+    }
   }
-  if (beads_in_smem) add(&SweepShape::rel_in_smem, 1);
-  const size_t smem = SweepSmem::make(shape).total;
-  if (csize > 1) {
-    // the cluster must be schedulable: csize CTAs of this size in one GPC
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(csize);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg);
-    if (e != cudaSuccess || clusters < 1)
-      return set_error(REMC_ERR_INVALID, "a cluster of %d sweep CTAs does not fit: %s", csize,
-                       cudaGetErrorString(e));
-    h->sweep_cluster_slots = clusters;
-  }
+  h->sweep_cluster_slots = clusters;
   if (ensure_sweep_scratch(h, shape)) return REMC_ERR_NOMEM;
   h->sweep_shape = shape;
   h->sweep_threads = threads;
@@ -1526,7 +1559,7 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   A.inst_list = inst_list;
   // a cluster schedule runs one cluster per replica (no work queue); the
   // one-replica-per-launch path always runs single CTAs
-  const int csize = persistent ? h->sweep_csize : 1;
+  const int csize = persistent ? h->sweep_shape.csize : 1;
   if (csize > 1) persistent = false;
   A.queue = persistent ? h->d_queue : nullptr;
   A.n_list = n_blocks;
@@ -1564,7 +1597,7 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   A.rec_stride = (int)h->recs_cap;
   A.rec_offset = rec_offset;
   A.n_steps = n_steps;
-  A.shape = csize == h->sweep_csize
+  A.shape = csize == h->sweep_shape.csize
                 ? h->sweep_shape
                 : base_shape(h, h->sweep_threads, h->mol_in_smem, csize, h->beads_in_smem);
   A.scratch = h->d_sweep_scratch;
@@ -1746,6 +1779,17 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
     h->lmax = std::max(h->lmax, lmax);
     for (int m = 0; m < d.n_mol; ++m)
       if (d.mol_start[m + 1] - d.mol_start[m] > 1) h->nrel = std::max(h->nrel, d.mol_start[m + 1]);
+    double pairs = 0.0;
+    int several = 0;
+    for (int m = 0; m < d.n_mol; ++m) {
+      const double n = d.mol_start[m + 1] - d.mol_start[m];
+      if (n > 1) {
+        pairs += n * (d.n_beads - n);
+        ++several;
+      }
+      h->any_crowders = h->any_crowders || d.mol_role[m] == -1;
+    }
+    if (several) h->chain_step_pairs = std::max(h->chain_step_pairs, pairs / several);
   }
   if (bead_cursor >= (size_t)1 << 31) {
     delete h;
@@ -2169,7 +2213,7 @@ int remc_sweep_plain(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0)
   int rc = check_ready(h);
   if (rc) return rc;
   if (n_steps < 0) return set_error(REMC_ERR_INVALID, "n_steps < 0");
-  if (h->sweep_csize > 1) {  // single CTAs all the same
+  if (h->sweep_shape.csize > 1) {  // single CTAs all the same
     rc = ensure_sweep_scratch(h, base_shape(h, h->sweep_threads, h->mol_in_smem, 1, h->beads_in_smem));
     if (rc) return rc;
   }

@@ -80,17 +80,24 @@ struct SweepShape {
   int nmax, mmax, lmax;  // beads, molecules, beads of the longest molecule
   int nrel;              // beads up to the last one of a molecule of several
   int csize;             // CTAs per replica (a thread-block cluster), 1, 2, 4 or 8
-  int vthreads;          // virtual threads per CTA: the schedule's threads per replica
+  // virtual threads, which fix the order of the sums: vsize (1 or csize) times
+  // vthreads, the schedule's CTAs and threads per replica
+  int vthreads, vsize;
   int mol_in_smem;       // molecule centres in shared memory (else in global memory)
   int beads_in_smem;     // beads and trial buffers in shared memory (else in global memory)
   int aj_in_smem;        // a chain step's sums per bead in shared memory
   int rel_in_smem;       // positions relative to the centres in shared memory
   int term_cap;          // terms of a chain step's split passes (0: no split passes)
 };
-// beads a CTA of the replica evaluates in a chain step, rounded up to whole rows
+// A chain step's sums a CTA holds: those of its own beads, rounded up to whole
+// rows, where CTAs and virtual CTAs are the same; else (a replica of one virtual
+// CTA on a cluster) those of all beads, in two buffers
 __host__ __device__ inline int local_beads(const SweepShape& s) {
-  const int g = s.vthreads * s.csize;
+  const int g = s.vthreads * s.vsize;
   return (s.nmax + g - 1) / g * s.vthreads;
+}
+__host__ __device__ inline int held_sums(const SweepShape& s) {
+  return local_beads(s) * (s.csize > s.vsize ? 2 : 1);
 }
 
 struct SweepArgs {
@@ -156,7 +163,7 @@ struct SweepSmem {
     s.ring = take(off, sizeof(StepRec) * kRing);
     // two buffers in a cluster, where another CTA may still read the last pass's
     s.sums = take(off, sizeof(double) * (p.csize > 1 ? 2 : 1) * pass_sums(p.csize));
-    s.aj = take(off, p.aj_in_smem ? sizeof(float) * local_beads(p) : 0);
+    s.aj = take(off, p.aj_in_smem ? sizeof(float) * held_sums(p) : 0);
     s.rel = take(off, p.rel_in_smem ? sizeof(float4) * p.nrel : 0);
     s.terms = take(off, sizeof(float) * p.term_cap);
     s.total = off;
@@ -398,6 +405,11 @@ __device__ __forceinline__ float wall_term(float2 r2, float A, float cut2, bool 
   return (LAST && last) ? __fmaf_rn(t.x, i6.x, -e.y) : d;
 }
 
+// A trial entry's last word: its bead's row of the type table, and whether the
+// row holds charges (a residue type without one needs no Debye-Hueckel terms:
+// 16 of the 20, 8 of some 60 issue slots of a pair).
+constexpr int kRowCharged = 1 << 16, kRowMask = kRowCharged - 1;
+
 // a_j of NJ beads per lane over the moved beads [k0, k1); with `terms` (NJ = 1)
 // the terms themselves go to terms[0], terms[stride], ...
 template <bool R12, bool CUT, bool FOLD, bool KH, int NJ, bool LAST, bool TERMS>
@@ -415,29 +427,62 @@ __device__ __forceinline__ void chain_terms(const float4* tp, int k0, int k1, co
     tj[q] = bead_type(pj[q].w);
     if constexpr (!TERMS) a[q] = 0.0f;
   }
-#pragma unroll 2
-  for (int k = k0; k < k1; ++k) {
-    const float4 P = tp[2 * k], Q = tp[2 * k + 1];
-    const float2 kx = make_float2(P.x, P.y), ky = make_float2(P.z, P.w), kz = make_float2(Q.x, Q.y);
-    const float4* row = s_tab + __float_as_int(Q.w);
+  // two moved beads at a time, so that their chains of operations overlap
+  auto step = [&](auto two, int k) {
+    constexpr int NK = decltype(two)::value ? 2 : 1;
+    float2 kx[NK], ky[NK], kz[NK];
+    int off[NK], any = 0;
+    float d[NK][NJ];
 #pragma unroll
-    for (int q = 0; q < NJ; ++q) {
-      const float2 r2 = pair_r2_2<FOLD>(kx, ky, kz, nx[q], ny[q], nz[q], B);
-      float d;
-      if constexpr (KH) {
-        const float2 e = kh_energy2(r2, row[tj[q]], c_xi);
-        d = __fsub_rn(e.x, e.y);
-      } else {
-        d = wall_term<R12, CUT, LAST>(r2, row[tj[q]].x, cut2, last[q]);
-      }
-      if constexpr (TERMS) {
-        *terms = d;
-        terms += stride;
-      } else {
-        a[q] += d;
-      }
+    for (int i = 0; i < NK; ++i) {
+      const float4 P = tp[2 * (k + i)], Q = tp[2 * (k + i) + 1];
+      kx[i] = make_float2(P.x, P.y);
+      ky[i] = make_float2(P.z, P.w);
+      kz[i] = make_float2(Q.x, Q.y);
+      off[i] = __float_as_int(Q.w);
+      any |= off[i];
     }
-  }
+    auto residues = [&](auto charged) {
+#pragma unroll
+      for (int i = 0; i < NK; ++i)
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) {
+          const float2 e = kh_energy2<decltype(charged)::value>(
+              pair_r2_2<FOLD>(kx[i], ky[i], kz[i], nx[q], ny[q], nz[q], B),
+              s_tab[(off[i] & kRowMask) + tj[q]], c_xi);
+          d[i][q] = __fsub_rn(e.x, e.y);
+        }
+    };
+    if constexpr (KH) {
+      // the same for every lane where the lanes share their moved beads
+      if (TERMS || (any & kRowCharged))
+        residues(std::true_type{});
+      else
+        residues(std::false_type{});
+    } else {
+#pragma unroll
+      for (int i = 0; i < NK; ++i)
+#pragma unroll
+        for (int q = 0; q < NJ; ++q)
+          d[i][q] = wall_term<R12, CUT, LAST>(
+              pair_r2_2<FOLD>(kx[i], ky[i], kz[i], nx[q], ny[q], nz[q], B),
+              s_tab[(off[i] & kRowMask) + tj[q]].x, cut2, last[q]);
+    }
+#pragma unroll
+    for (int i = 0; i < NK; ++i)
+#pragma unroll
+      for (int q = 0; q < NJ; ++q) {
+        if constexpr (TERMS) {
+          *terms = d[i][q];
+          terms += stride;
+        } else {
+          a[q] += d[i][q];
+        }
+      }
+  };
+  int k = k0;
+  for (; k + 2 <= k1; k += 2) step(std::true_type{}, k);
+  if (k < k1) step(std::false_type{}, k);
 }
 
 // One CTA (or cluster of csize CTAs) per replica-instance, persistent over the
@@ -446,10 +491,11 @@ __device__ __forceinline__ void chain_terms(const float4* tp, int k0, int k1, co
 // one other step; its installs are behind a barrier when the next pass begins,
 // so any thread may read any bead.
 // In a cluster every CTA holds the whole replica and takes every step: the work
-// is split over the cluster's warps (groups) or beads (chain steps: CTA r
-// evaluates j with j / vthreads = r mod csize), the sums go to every CTA's
-// shared memory and one cluster barrier per pass shows them; every CTA then
-// decides and installs the same. Rank 0 alone writes state that is not
+// is split over the cluster's warps (groups) or beads (chain steps: with csize
+// virtual CTAs, CTA r evaluates the beads of its own virtual threads and the
+// virtual warps' sums go to every CTA's shared memory; with one, it evaluates a
+// part of the list and the sums per bead go there). One cluster barrier per
+// pass shows the sums; every CTA then decides and installs the same. Rank 0 alone writes state that is not
 // idempotent (rotations, counters, samples) and the final state.
 // GB: the beads stay where they are in global memory (updated in place, no
 // prologue copy and no write-back), the trial buffers in global scratch; every
@@ -461,6 +507,7 @@ template <bool R12, bool CUT, bool FOLD, bool CLUSTER, bool GB>
 __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SweepSmem L = SweepSmem::make(A.shape);
+  const int held = local_beads(A.shape);
   float4* const s_tab = reinterpret_cast<float4*>(smem_raw + L.tab);
   StepRec* const s_ring = reinterpret_cast<StepRec*>(smem_raw + L.ring);
   double* const s_sums = reinterpret_cast<double*>(smem_raw + L.sums);
@@ -474,9 +521,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   constexpr unsigned full = 0xffffffffu;
   const int csize = CLUSTER ? A.shape.csize : 1;
   const int crank = CLUSTER ? (int)cooperative_groups::this_cluster().block_rank() : 0;
-  // virtual threads: vthr of this CTA, gstride of the replica (powers of two)
-  const int vthr = A.shape.vthreads;
-  const int gstride = vthr * csize, gmask = gstride - 1;
+  // virtual threads: vthr of a virtual CTA, gstride of the replica (powers of two)
+  const int vthr = A.shape.vthreads, vsize = CLUSTER ? A.shape.vsize : 1;
+  const int vrank = vsize > 1 ? crank : 0;
+  const bool spread = CLUSTER && vsize < csize;  // one virtual CTA on a cluster
+  const int gstride = vthr * vsize, gmask = gstride - 1;
   const int lgv = 31 - __clz(vthr), lgs = 31 - __clz(gstride);
   // warps of the replica, real and virtual
   const int lg_warps = 31 - __clz(nwarps * csize), lg_vwarps = lgs - 5;
@@ -526,12 +575,21 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   float4* const s_tpos = GB ? scratch : reinterpret_cast<float4*>(smem_raw + L.trial_pos);
   float4* const s_trel =
       GB ? scratch + 2 * A.shape.lmax : reinterpret_cast<float4*>(smem_raw + L.trial_rel);
-  float* const s_aj = A.shape.aj_in_smem ? reinterpret_cast<float*>(smem_raw + L.aj)
-                                         : reinterpret_cast<float*>(scratch + 3 * A.shape.lmax);
+  float* const sums_aj = A.shape.aj_in_smem ? reinterpret_cast<float*>(smem_raw + L.aj)
+                                            : reinterpret_cast<float*>(scratch + 3 * A.shape.lmax);
   float4* const rel =
       A.shape.rel_in_smem ? reinterpret_cast<float4*>(smem_raw + L.rel) : A.rel + bead_off;
   float4* const cent = A.shape.mol_in_smem ? reinterpret_cast<float4*>(smem_raw + L.centres)
                                            : A.centre + mol_off;
+
+  // residue types with charges, by the type table
+  unsigned charged;
+  {
+    bool any = false;
+    if (lane < kNumAmino)
+      for (int t = 0; t < kNumAmino; ++t) any = any || A.tab[lane * kNT + t].w != 0.0f;
+    charged = __ballot_sync(full, any);
+  }
 
   // ---- prologue: make the instance resident in shared memory
   for (int i = tid; i < kNT * kNT; i += nthr) s_tab[i] = A.tab[i];
@@ -690,7 +748,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   int avail = min(kRing, n_steps), filled = avail;
   int parity = 0;      // buffer of this pass's sums (clusters alternate)
   bool alone = false;  // the next step's sum does not split: taken like a chain step
-  if (n_steps > 0) look(0, avail, to_sample);
+  if (ncb < N && n_steps > 0) look(0, avail, to_sample);  // without crowders run stays zero
   for (int s = 0; s < n_steps;) {
     if (filled == avail && filled < n_steps && s >= filled - 32) {
       const int nrec = min(32, n_steps - filled);
@@ -707,6 +765,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (alone) run = 0;
     alone = false;
     double* const sums = s_sums + parity * pass_sums(csize);
+    float* const s_aj = sums_aj + (spread && parity ? held : 0);
     if (CLUSTER) parity ^= 1;
 
     if (run > 0) {
@@ -899,38 +958,46 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
         const float4 np = make_float4(__fadd_rn(rl.x, c_new.x), __fadd_rn(rl.y, c_new.y),
                                       __fadd_rn(rl.z, c_new.z), ol.w);
         s_tpos[2 * k] = make_float4(np.x, ol.x, np.y, ol.y);
-        s_tpos[2 * k + 1] = make_float4(np.z, ol.z, ol.w, __int_as_float(bead_type(ol.w) * kNT));
+        s_tpos[2 * k + 1] = make_float4(np.z, ol.z, ol.w, __int_as_float((bead_type(ol.w) * kNT) |
+                                                         (((charged >> bead_type(ol.w)) & 1u) ? kRowCharged : 0)));
       }
     }
     __syncthreads();  // trial positions
     // records this pass waits for are not readable yet: a shorter run
-    if (s + 1 < n_steps)
+    if (ncb < N && s + 1 < n_steps)
       look(s + 1, avail, to_sample <= 0 ? 0 : to_sample == 1 ? A.sample_every : to_sample - 1);
 
     // ---- a_j of the beads outside the molecule, residue pairs then crowder pairs
     if (!skip) {
       const PackedBox PB = packed_box(box, invbox);
       const float cut2 = s_tab[(kNT - 1) * kNT].z;
-      // bead of place x of a list that starts at place x0 of this CTA's beads,
-      // its place y among them, and whether it counts. A single CTA's list
-      // leaves the molecule out; in a cluster its places are masked
+      // bead at place x of the list of beads, the place y of its sum, and whether
+      // it counts. With one virtual CTA the list leaves the molecule out; else
+      // it holds this CTA's beads, the molecule's masked
       auto bead_at = [&](int x, int& y, bool& counts) {
         int j;
-        if (!CLUSTER) {
+        if (!CLUSTER || spread) {
           j = x < m0 ? x : x + n;
           y = j;
           counts = true;
         } else {
           y = x;
-          j = ((x >> lgv) << lgs) + crank * vthr + (x & (vthr - 1));
+          j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
           counts = (unsigned)(j - m0) >= (unsigned)n;
         }
         return j;
       };
-      // places of this CTA's beads below bead e
+      // places of the list below bead e
       auto places = [&](int e) {
-        if (!CLUSTER) return e <= m0 ? e : max(m0, e - n);
-        return ((e >> lgs) << lgv) + min(max((e & gmask) - crank * vthr, 0), vthr);
+        if (!CLUSTER || spread) return e <= m0 ? e : max(m0, e - n);
+        return ((e >> lgs) << lgv) + min(max((e & gmask) - vrank * vthr, 0), vthr);
+      };
+      auto put_sum = [&](int y, float a) {
+        if (spread)
+          for (int k = 0; k < csize; ++k)
+            cooperative_groups::this_cluster().map_shared_rank(s_aj, k)[y] = a;
+        else
+          s_aj[y] = a;
       };
       // is crowder pair j the odd one of its virtual thread's last pass (see
       // wall_term)? Alone in a pass: a one-residue chain's pairs, and the
@@ -940,8 +1007,13 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
         const int a = j < m0 ? ncb : max(m0 + n, ncb), e = j < m0 ? m0 : N;
         return j + gstride >= e && ((((j - a) >> lgs) & 1) == 0);
       };
-      auto run_class = [&](auto kh, int x, const int end) {
+      auto run_class = [&](auto kh, int x, int end) {
         constexpr bool KH = decltype(kh)::value;
+        if (spread) {  // this CTA's part of the list
+          const int part = (end - x + csize - 1) / csize;
+          x = min(x + crank * part, end);
+          end = min(x + part, end);
+        }
         // one or two beads per lane, all moved beads
         auto whole = [&](auto two) {
           constexpr int NJ = decltype(two)::value ? 2 : 1;
@@ -967,7 +1039,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
                                                                     A.K.c_xi, cut2, a, nullptr, 0);
 #pragma unroll
           for (int q = 0; q < NJ; ++q)
-            if (put[q]) s_aj[y[q]] = a[q];
+            if (put[q]) put_sum(y[q], a[q]);
         };
         const int cap = A.shape.term_cap;
         // two beads per lane while that keeps most threads at work, then one;
@@ -979,7 +1051,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
             whole(std::false_type{});
           x += 2 * nthr;
         }
-        while (end - x > (cap ? nthr - nthr / 4 : 0)) {
+        while (end - x > min(nthr - nthr / 4, cap / 8)) {
           if (x + warp * 32 < end) whole(std::false_type{});
           x += nthr;
         }
@@ -987,44 +1059,65 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
         // the moved beads, leave the terms, and one adds them in order
         const int rest = end - x;
         if (rest > 0) {
-          const int part = __float2int_rd(((float)tid + 0.5f) / (float)rest);  // tid / rest
-          const int parts = __float2int_rd(((float)nthr + 0.5f) / (float)rest);
+          // quotients of small integers: the half keeps them off the roundings
+          auto quotient = [](int a, int b) { return __float2int_rd(((float)a + 0.5f) * fast_rcp((float)b)); };
+          const int part = quotient(tid, rest), parts = quotient(nthr, rest);
           int y;
           bool put;
           const int j = bead_at(x + tid - part * rest, y, put);
           const float4 pj = s_beads[j];
           const bool last = !KH && !CUT && odd_last(j);
-          const int most = cap / rest;  // moved beads per round
+          const int most = (cap / rest) & ~7;  // moved beads per round
           float a = 0.0f;
           for (int k0 = 0; k0 < n; k0 += most) {
             const int nk = min(most, n - k0);
-            const int per = __float2int_ru((float)nk / (float)parts);
+            const int per = quotient(nk + parts - 1, parts);
             const int ka = min(part * per, nk), kb = min(ka + per, nk);
+            // whole eights: terms past the last moved bead are zero
+            for (int e = nk * rest + tid; e < ((nk + 7) & ~7) * rest; e += nthr) s_terms[e] = 0.0f;
             if (part < parts)
               chain_terms<R12, CUT, FOLD, KH, 1, !KH && !CUT, true>(
                   s_tpos, k0 + ka, k0 + kb, s_tab, &pj, &last, PB, A.K.c_xi, cut2, nullptr,
                   s_terms + ka * rest + tid - part * rest, rest);
             __syncthreads();
-            if (tid < rest) {
-#pragma unroll 8
-              for (int k = 0; k < nk; ++k) a += s_terms[k * rest + tid];
+            if (tid < rest) {  // eight terms ahead of the chain of additions
+              const float* t = s_terms + tid;
+              float now[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q) now[q] = t[q * rest];
+              for (int k = 8; k < nk; k += 8) {
+                t += 8 * rest;
+                float next[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) next[q] = t[q * rest];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                  a += now[q];
+                  now[q] = next[q];
+                }
+              }
+#pragma unroll
+              for (int q = 0; q < 8; ++q) a += now[q];
             }
             __syncthreads();
           }
-          if (tid < rest && put) s_aj[y] = a;
+          if (tid < rest && put) put_sum(y, a);
         }
       };
       const int xk = crowd ? 0 : places(ncb), xe = places(N);
       run_class(std::true_type{}, 0, xk);
       run_class(std::false_type{}, xk, xe);
     }
-    __syncthreads();  // every a_j
+    if (spread)  // every a_j
+      cluster_barrier();
+    else
+      __syncthreads();
 
     // ---- virtual threads' sums, virtual warps' FP64 sums, one fixed tree
     double d_all = 0.0, d_cc = 0.0;
     if (!skip && tid < vthr) {
       float acc_c = 0.0f, acc_o = 0.0f;
-      for (int j = crank * vthr + tid, y = tid; j < N; j += gstride, y += vthr) {
+      for (int j = vrank * vthr + tid, y = tid; j < N; j += gstride, y += vthr) {
         if ((unsigned)(j - m0) < (unsigned)n) continue;
         const float a = s_aj[y];
         if (j < ncb && !crowd)
@@ -1036,28 +1129,28 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       d_all = (double)acc_o;
     }
     if (warp < 8) {
-      if (32 * warp < vthr) {
-        d_all = warp_sum(d_all);
-        d_cc = warp_sum(d_cc);
-      }
-      if (lane == 0)
-        for (int k = 0; k < csize; ++k) {
+      // sums of d_all in lanes 0-15, of d_cc in 16-31, each in warp_sum's order;
+      // zero for virtual warps there are none of
+      double v = 0.0;
+      if (32 * warp < vthr) v = warp_sum_split(d_all, d_cc, lane);
+      if ((lane & 15) == 0)
+        for (int k = 0; k < vsize; ++k) {
           double* dst = sums;
-          if (CLUSTER) dst = cooperative_groups::this_cluster().map_shared_rank(sums, k);
-          for (int w = warp; w < 8; w += nwarps) {  // virtual warps there are none of: zero
-            dst[16 * crank + w] = w == warp ? d_all : 0.0;
-            dst[16 * crank + 8 + w] = w == warp ? d_cc : 0.0;
-          }
+          if (CLUSTER && !spread) dst = cooperative_groups::this_cluster().map_shared_rank(sums, k);
+          dst[16 * vrank + (lane >> 1) + warp] = v;
         }
     }
     if (landing) cp_async_wait_all();
-    cluster_barrier();
+    if (spread)
+      __syncthreads();
+    else
+      cluster_barrier();
     if (landing) avail = filled;
 
     // ---- every thread takes the same decision
     double dE = tree_sum8(sums), dE_cc = 0.0;
     if (!crowd) dE_cc = tree_sum8(sums + 8);
-    for (int k = 1; k < csize; ++k) {  // the other CTAs' sums, in rank order
+    for (int k = 1; k < vsize; ++k) {  // the other CTAs' sums, in rank order
       dE += tree_sum8(sums + 16 * k);
       if (!crowd) dE_cc += tree_sum8(sums + 16 * k + 8);
     }
