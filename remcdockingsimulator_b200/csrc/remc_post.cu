@@ -1,5 +1,5 @@
 // Batched post-processing (include/remc_post.h): pose reconstruction of bound
-// conformations and DRMS against a reference conformation, one CTA per frame.
+// conformations and DRMS against a reference conformation.
 //
 // Reconstruction follows pdbgen (post processor/pdbgensrc/pdbgen.cpp:166-215)
 // in the reference's precisions: the pose quaternion is normalised twice in
@@ -10,12 +10,14 @@
 // intrinsics, so the result is bit-identical to the host arithmetic.
 //
 // DRMS follows drms.cpp:7-57 (FP32 Vector3f::magnitude of the FP32 difference,
-// |d_sim - d_ref| in FP32, summed in FP64); each thread sums the pairs of its
-// i beads and the CTA adds the per-thread sums in a fixed order.
+// |d_sim - d_ref| in FP32, summed in FP64); the lanes' sums are added in a fixed
+// order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 
 #include "../../include/remc_b200.h"
@@ -90,93 +92,176 @@ __global__ void rebuild_kernel(const float* __restrict__ rel0, const int* __rest
   }
 }
 
-// |a - b| as Vector3f::magnitude computes it: FP32 squares summed left to
-// right, FP32 square root.
-__device__ __forceinline__ float dist3(const float* a, const float* b) {
-  const float dx = __fsub_rn(a[0], b[0]), dy = __fsub_rn(a[1], b[1]), dz = __fsub_rn(a[2], b[2]);
+// The length of (dx, dy, dz) as Vector3f::magnitude computes it: FP32 squares
+// summed left to right, FP32 square root.
+__device__ __forceinline__ float length3(float dx, float dy, float dz) {
   return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+}
+__device__ __forceinline__ float dist3(const float* a, const float* b) {
+  return length3(__fsub_rn(a[0], b[0]), __fsub_rn(a[1], b[1]), __fsub_rn(a[2], b[2]));
 }
 
 constexpr int kDrmsThreads = 256;
+constexpr int kDrmsFrames = 4;  // frames a CTA takes against one evaluation of the reference
 
+// Per (group of kDrmsFrames frames, part of the i beads): a warp takes one bead
+// i at a time and its lanes the beads j of later molecules, side by side. A
+// reference distance (two with REVERSE) serves all frames of the group. The
+// frames sit in shared memory by coordinate (SHARED; frames too large for it
+// are read from global memory). Bound by the square roots: 4 chains of 150, 500
+// frames, both orders, ran 378 us with one CTA per frame, a thread per bead i
+// and both distances evaluated per frame and pair.
+// out[frame][part]: sums; counts[frame][part]: native, recovered, binding pairs.
+struct DrmsOut {
+  double a, b;
+  unsigned long long native, recovered, binding;
+};
+template <bool REVERSE, bool SHARED>
 __global__ void __launch_bounds__(kDrmsThreads) drms_kernel(
-    const float* __restrict__ frames, const float* __restrict__ ref, const int* __restrict__ ms,
-    const int* __restrict__ mol_of, int n_mol, int n_beads, int reverse, float native_cut,
-    float recovered_cut, double* __restrict__ drms, double* __restrict__ drms_rev,
-    unsigned long long* __restrict__ counts) {
-  __shared__ double s_a[kDrmsThreads], s_b[kDrmsThreads];
-  __shared__ unsigned long long s_c[3][kDrmsThreads];
-  const int f = blockIdx.x, tid = threadIdx.x;
-  const float* x = frames + (size_t)f * n_beads * 3;
-  double sa = 0.0, sb = 0.0;
-  unsigned long long cn = 0, cr = 0, cb = 0;
-  for (int i = tid; i < n_beads; i += kDrmsThreads) {
+    const float* __restrict__ frames, int n_frames, const float* __restrict__ ref,
+    const int* __restrict__ ms, const int* __restrict__ mol_of, int n_beads, float native_cut,
+    float recovered_cut, DrmsOut* __restrict__ out) {
+  extern __shared__ float s_x[];  // [frame][coordinate][bead]
+  __shared__ DrmsOut s_out[kDrmsThreads / 32][kDrmsFrames];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int f0 = blockIdx.x * kDrmsFrames, nf = min(kDrmsFrames, n_frames - f0);
+  const float* x = frames + (size_t)f0 * n_beads * 3;
+  if (SHARED) {
+    for (int e = tid; e < nf * n_beads * 3; e += kDrmsThreads) {
+      const int bead = e / 3, f = bead / n_beads;
+      s_x[(3 * f + e - 3 * bead) * n_beads + bead - f * n_beads] = x[e];
+    }
+    __syncthreads();
+  }
+  auto at = [&](int f, int c, int bead) {
+    return SHARED ? s_x[(3 * f + c) * n_beads + bead] : x[((size_t)f * n_beads + bead) * 3 + c];
+  };
+  double sa[kDrmsFrames] = {}, sb[kDrmsFrames] = {};
+  unsigned cn = 0, cr[kDrmsFrames] = {}, cb[kDrmsFrames] = {};
+  const int warps = (kDrmsThreads / 32) * gridDim.y;
+  for (int i = blockIdx.y * (kDrmsThreads / 32) + warp; i < n_beads; i += warps) {
     const int I = mol_of[i], li = i - ms[I];
-    for (int j = ms[I + 1]; j < n_beads; ++j) {  // beads of molecules J > I
-      const float ds = dist3(x + 3 * i, x + 3 * j);
+    float xi[kDrmsFrames][3];
+#pragma unroll
+    for (int f = 0; f < kDrmsFrames; ++f)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) xi[f][c] = at(min(f, nf - 1), c, i);
+    for (int j = ms[I + 1] + lane; j < n_beads; j += 32) {  // beads of molecules J > I
       const float de = dist3(ref + 3 * i, ref + 3 * j);
-      sa += (double)fabsf(__fsub_rn(ds, de));
-      cn += de < native_cut ? 1ull : 0ull;
-      cr += (de < native_cut && ds < recovered_cut) ? 1ull : 0ull;
-      cb += ds < native_cut ? 1ull : 0ull;
-      if (reverse) {
+      float dr = 0.0f;
+      if (REVERSE) {
         // drms.cpp:45-46: the reference's molecules I and J swapped
         const int J = mol_of[j], lj = j - ms[J];
-        const float dr = dist3(ref + 3 * (ms[J] + li), ref + 3 * (ms[I] + lj));
-        sb += (double)fabsf(__fsub_rn(ds, dr));
+        dr = dist3(ref + 3 * (ms[J] + li), ref + 3 * (ms[I] + lj));
+      }
+      const bool near = de < native_cut;
+      cn += near;
+#pragma unroll
+      for (int f = 0; f < kDrmsFrames; ++f) {
+        const int g = min(f, nf - 1);  // past the last frame: repeated, not written out
+        const float ds = length3(__fsub_rn(xi[f][0], at(g, 0, j)), __fsub_rn(xi[f][1], at(g, 1, j)),
+                                 __fsub_rn(xi[f][2], at(g, 2, j)));
+        sa[f] += (double)fabsf(__fsub_rn(ds, de));
+        if (REVERSE) sb[f] += (double)fabsf(__fsub_rn(ds, dr));
+        cr[f] += near && ds < recovered_cut;
+        cb[f] += ds < native_cut;
       }
     }
   }
-  s_a[tid] = sa;
-  s_b[tid] = sb;
-  s_c[0][tid] = cn;
-  s_c[1][tid] = cr;
-  s_c[2][tid] = cb;
+  auto total = [](unsigned v) {  // 64 bits: a warp may meet 2^32 pairs
+    unsigned long long t = v;
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    return t;
+  };
+#pragma unroll
+  for (int f = 0; f < kDrmsFrames; ++f) {
+    DrmsOut o;
+    o.a = warp_sum(sa[f]);
+    o.b = REVERSE ? warp_sum(sb[f]) : 0.0;
+    o.native = total(cn);
+    o.recovered = total(cr[f]);
+    o.binding = total(cb[f]);
+    if (lane == 0) s_out[warp][f] = o;
+  }
   __syncthreads();
-  if (tid == 0) {
-    double a = 0.0, b = 0.0;
-    unsigned long long c[3] = {0, 0, 0};
-    for (int t = 0; t < kDrmsThreads; ++t) {
-      a += s_a[t];
-      b += s_b[t];
-      for (int k = 0; k < 3; ++k) c[k] += s_c[k][t];
+  if (tid < nf) {
+    DrmsOut t = s_out[0][tid];
+    for (int w = 1; w < kDrmsThreads / 32; ++w) {
+      const DrmsOut o = s_out[w][tid];
+      t.a += o.a;
+      t.b += o.b;
+      t.native += o.native;
+      t.recovered += o.recovered;
+      t.binding += o.binding;
     }
-    drms[f] = a;
-    drms_rev[f] = b;
-    for (int k = 0; k < 3; ++k) counts[3 * f + k] = c[k];
+    out[(size_t)(f0 + tid) * gridDim.y + blockIdx.y] = t;
   }
 }
 
+// One slab of device memory for a call, from a pool per device that keeps up to
+// kPoolKeep bytes between calls (the rest goes back to the driver at the next
+// synchronisation). Seven allocations and frees of their own had taken most of
+// a call on 1000 small frames. Stream-ordered on the legacy default stream, on
+// which the calls run, so several host threads may use it at once.
+constexpr size_t kPoolKeep = (size_t)64 << 20;
+class Slab {
+ public:
+  ~Slab() {
+    if (base_) cudaFreeAsync(base_, 0);
+  }
+  // offsets first (take), then the memory (get)
+  size_t take(size_t bytes) {
+    const size_t at = size_;
+    size_ += (bytes + 255) & ~(size_t)255;
+    return at;
+  }
+  int get() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+      return fail(REMC_ERR_CUDA, "post: no current device");
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      if (!pools_[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess)
+          return fail(REMC_ERR_NOMEM, "post: no memory pool");
+        unsigned long long keep = kPoolKeep;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools_[dev] = pool;
+      }
+    }
+    if (cudaMallocFromPoolAsync((void**)&base_, size_ ? size_ : 1, pools_[dev], 0) != cudaSuccess) {
+      base_ = nullptr;
+      cudaGetLastError();
+      return fail(REMC_ERR_NOMEM, "post: device allocation failed");
+    }
+    return REMC_OK;
+  }
+  template <class T>
+  T* at(size_t offset) const {
+    return reinterpret_cast<T*>(base_ + offset);
+  }
+
+ private:
+  static constexpr int kMaxDevices = 64;
+  static std::mutex mutex_;
+  static cudaMemPool_t pools_[kMaxDevices];
+  unsigned char* base_ = nullptr;
+  size_t size_ = 0;
+};
+std::mutex Slab::mutex_;
+cudaMemPool_t Slab::pools_[Slab::kMaxDevices] = {};
+
 template <class T>
-int to_device(T** d, const T* h, size_t n) {
-  if (cudaMalloc((void**)d, sizeof(T) * (n ? n : 1)) != cudaSuccess)
-    return fail(REMC_ERR_NOMEM, "post: device allocation failed");
-  if (n && cudaMemcpy(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice) != cudaSuccess)
+int copy_in(T* d, const T* h, size_t n) {
+  if (n && cudaMemcpyAsync(d, h, sizeof(T) * n, cudaMemcpyHostToDevice, 0) != cudaSuccess)
     return fail(REMC_ERR_CUDA, "post: host to device copy failed");
   return REMC_OK;
 }
-
-struct DevBufs {
-  std::vector<void*> p;
-  ~DevBufs() {
-    for (void* q : p) cudaFree(q);
-  }
-  template <class T>
-  int up(T** d, const T* h, size_t n) {
-    *d = nullptr;
-    int rc = to_device(d, h, n);
-    if (*d) p.push_back(*d);
-    return rc;
-  }
-  template <class T>
-  int alloc(T** d, size_t n) {
-    *d = nullptr;
-    if (cudaMalloc((void**)d, sizeof(T) * (n ? n : 1)) != cudaSuccess)
-      return fail(REMC_ERR_NOMEM, "post: device allocation failed");
-    p.push_back(*d);
-    return REMC_OK;
-  }
-};
 
 int check_starts(const int* mol_start, int n_mol) {
   if (!mol_start || n_mol <= 0 || mol_start[0] != 0)
@@ -201,25 +286,28 @@ int remc_post_rebuild(const float* rel0, const int* mol_start, int n_mol, const 
   if (!(box > 0.0f) || !std::isfinite(box)) return fail(REMC_ERR_INVALID, "post_rebuild: bad box");
   if (n_frames == 0) return REMC_OK;
   const int nb = mol_start[n_mol];
-  DevBufs B;
-  float *d_rel, *d_cen, *d_pos, *d_cout = nullptr;
-  int *d_ms, *d_shift;
-  double* d_q;
-  if ((rc = B.up(&d_rel, rel0, 3 * (size_t)nb)) || (rc = B.up(&d_ms, mol_start, n_mol + 1)) ||
-      (rc = B.up(&d_shift, shift, n_mol)) || (rc = B.up(&d_q, quat, 4 * (size_t)n_mol * n_frames)) ||
-      (rc = B.up(&d_cen, centre, 3 * (size_t)n_mol * n_frames)) ||
-      (rc = B.alloc(&d_pos, 3 * (size_t)nb * n_frames)))
+  const size_t nm = (size_t)n_mol * n_frames, np = (size_t)nb * n_frames;
+  Slab B;
+  const size_t o_rel = B.take(sizeof(float) * 3 * nb), o_ms = B.take(sizeof(int) * (n_mol + 1)),
+               o_shift = B.take(sizeof(int) * n_mol), o_q = B.take(sizeof(double) * 4 * nm),
+               o_cen = B.take(sizeof(float) * 3 * nm), o_pos = B.take(sizeof(float) * 3 * np),
+               o_cout = B.take(centre_out ? sizeof(float) * 3 * nm : 0);
+  if ((rc = B.get())) return rc;
+  float *d_rel = B.at<float>(o_rel), *d_cen = B.at<float>(o_cen), *d_pos = B.at<float>(o_pos),
+        *d_cout = centre_out ? B.at<float>(o_cout) : nullptr;
+  int *d_ms = B.at<int>(o_ms), *d_shift = B.at<int>(o_shift);
+  double* d_q = B.at<double>(o_q);
+  if ((rc = copy_in(d_rel, rel0, 3 * (size_t)nb)) || (rc = copy_in(d_ms, mol_start, n_mol + 1)) ||
+      (rc = copy_in(d_shift, shift, n_mol)) || (rc = copy_in(d_q, quat, 4 * nm)) ||
+      (rc = copy_in(d_cen, centre, 3 * nm)))
     return rc;
-  if (centre_out && (rc = B.alloc(&d_cout, 3 * (size_t)n_mol * n_frames))) return rc;
   rebuild_kernel<<<n_frames, 256>>>(d_rel, d_ms, n_mol, d_shift,
                                     make_float3(centre0[0], centre0[1], centre0[2]), box, d_q,
                                     d_cen, nb, d_pos, d_cout);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpy(pos, d_pos, sizeof(float) * 3 * (size_t)nb * n_frames, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(pos, d_pos, sizeof(float) * 3 * np, cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && centre_out)
-    e = cudaMemcpy(centre_out, d_cout, sizeof(float) * 3 * (size_t)n_mol * n_frames,
-                   cudaMemcpyDeviceToHost);
+    e = cudaMemcpy(centre_out, d_cout, sizeof(float) * 3 * nm, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
     char msg[256];
     snprintf(msg, sizeof(msg), "post_rebuild: %s", cudaGetErrorString(e));
@@ -247,25 +335,42 @@ int remc_post_drms(const float* frames, int n_frames, const float* ref, const in
     for (int b = mol_start[m]; b < mol_start[m + 1]; ++b) mol_of[b] = m;
     n_pairs += (double)(mol_start[m + 1] - mol_start[m]) * (double)(nb - mol_start[m + 1]);
   }
-  DevBufs B;
-  float *d_x, *d_ref;
-  int *d_ms, *d_mol;
-  double *d_a, *d_b;
-  unsigned long long* d_c;
-  if ((rc = B.up(&d_x, frames, 3 * (size_t)nb * n_frames)) || (rc = B.up(&d_ref, ref, 3 * (size_t)nb)) ||
-      (rc = B.up(&d_ms, mol_start, n_mol + 1)) || (rc = B.up(&d_mol, mol_of.data(), (size_t)nb)) ||
-      (rc = B.alloc(&d_a, n_frames)) || (rc = B.alloc(&d_b, n_frames)) ||
-      (rc = B.alloc(&d_c, 3 * (size_t)n_frames)))
+  // groups of frames, and parts of the i beads where the groups are too few for
+  // the GPU (about two CTAs per SM)
+  int dev = 0, sms = 148, smem_max = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const int groups = (n_frames + kDrmsFrames - 1) / kDrmsFrames;
+  const int most = std::max(1, nb / (2 * (kDrmsThreads / 32)));
+  const int parts = std::max(1, std::min(most, (4 * sms + groups - 1) / groups));
+  const size_t smem = sizeof(float) * 3 * (size_t)nb * kDrmsFrames;
+  const bool shared = smem + 4096 <= (size_t)smem_max;
+  const size_t n_out = (size_t)n_frames * parts;
+  Slab B;
+  const size_t o_x = B.take(sizeof(float) * 3 * (size_t)nb * n_frames), o_ref = B.take(sizeof(float) * 3 * nb),
+               o_ms = B.take(sizeof(int) * (n_mol + 1)), o_mol = B.take(sizeof(int) * nb),
+               o_out = B.take(sizeof(DrmsOut) * n_out);
+  if ((rc = B.get())) return rc;
+  float *d_x = B.at<float>(o_x), *d_ref = B.at<float>(o_ref);
+  int *d_ms = B.at<int>(o_ms), *d_mol = B.at<int>(o_mol);
+  DrmsOut* d_out = B.at<DrmsOut>(o_out);
+  if ((rc = copy_in(d_ref, ref, 3 * (size_t)nb)) || (rc = copy_in(d_ms, mol_start, n_mol + 1)) ||
+      (rc = copy_in(d_mol, (const int*)mol_of.data(), (size_t)nb)) ||
+      (rc = copy_in(d_x, frames, 3 * (size_t)nb * n_frames)))
     return rc;
-  drms_kernel<<<n_frames, kDrmsThreads>>>(d_x, d_ref, d_ms, d_mol, n_mol, nb, reverse ? 1 : 0,
-                                          native_cut, recovered_cut, d_a, d_b, d_c);
-  std::vector<double> a(n_frames), b(n_frames);
-  std::vector<unsigned long long> c(3 * (size_t)n_frames);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpy(a.data(), d_a, sizeof(double) * n_frames, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(b.data(), d_b, sizeof(double) * n_frames, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(c.data(), d_c, sizeof(unsigned long long) * c.size(), cudaMemcpyDeviceToHost);
+  auto kernel = reverse ? (shared ? drms_kernel<true, true> : drms_kernel<true, false>)
+                        : (shared ? drms_kernel<false, true> : drms_kernel<false, false>);
+  cudaError_t e = cudaSuccess;
+  if (shared && smem > 48 * 1024)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  std::vector<DrmsOut> out(n_out);
+  if (e == cudaSuccess) {
+    kernel<<<dim3(groups, parts), kDrmsThreads, shared ? smem : 0>>>(
+        d_x, n_frames, d_ref, d_ms, d_mol, nb, native_cut, recovered_cut, d_out);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out.data(), d_out, sizeof(DrmsOut) * n_out, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
     char msg[256];
     snprintf(msg, sizeof(msg), "post_drms: %s", cudaGetErrorString(e));
@@ -273,12 +378,21 @@ int remc_post_drms(const float* frames, int n_frames, const float* ref, const in
   }
   for (int f = 0; f < n_frames; ++f) {
     // drms.cpp:32 and :52: drms /= N; reverse: min(drms, drms2 / N)
-    double d = a[f] / n_pairs;
-    if (reverse) d = std::min(d, b[f] / n_pairs);
+    DrmsOut t = out[(size_t)f * parts];
+    for (int p = 1; p < parts; ++p) {
+      const DrmsOut& o = out[(size_t)f * parts + p];
+      t.a += o.a;
+      t.b += o.b;
+      t.native += o.native;
+      t.recovered += o.recovered;
+      t.binding += o.binding;
+    }
+    double d = t.a / n_pairs;
+    if (reverse) d = std::min(d, t.b / n_pairs);
     drms[f] = d;
-    if (native) native[f] = (long long)c[3 * f];
-    if (recovered) recovered[f] = (long long)c[3 * f + 1];
-    if (binding) binding[f] = (long long)c[3 * f + 2];
+    if (native) native[f] = (long long)t.native;
+    if (recovered) recovered[f] = (long long)t.recovered;
+    if (binding) binding[f] = (long long)t.binding;
   }
   return REMC_OK;
 }
