@@ -1,12 +1,11 @@
 // Drop-in replacements for the reference's CUDA C ABI (include/remc_reference_abi.h),
 // in the reference's own device data layout.
 //
-// Energy: tiled upper-triangle pair sum. A persistent grid walks the
-// (i-tile, j-tile >= i-tile) items of 128 beads; each CTA stages the j-tile
-// (positions + metadata) in shared memory, each thread keeps one i bead in
-// registers, pair terms are FP32 (MUFU rsqrt/ex2) and each item's sum goes to
-// a per-item FP64 partial; a second kernel adds the partials in a fixed order
-// (deterministic result). Follows Replica::E (Replica.cpp:603-745) and the
+// Energy: tiled upper-triangle pair sum, one CTA per item of 128 beads i by 32
+// or 128 beads j; each CTA stages its beads j (positions + metadata) in shared
+// memory, each thread keeps one i bead in registers, pair terms are FP32 (MUFU
+// rsqrt/ex2) and each item's sum goes to a per-item FP64 partial; the last CTA
+// to finish adds the partials in a fixed order (deterministic result). Follows Replica::E (Replica.cpp:603-745) and the
 // reference kernel's masking rules (CudaFunctions.cu:483-548): padding beads
 // have position w < 0, beads of the same molecule share w, a pair involving a
 // crowder (metadata w = -1) is (6/r)^6 inside 15 A.
@@ -89,96 +88,156 @@ RefConsts make_consts(float* unscale = nullptr) {
   return C;
 }
 
-// Triangle index of item (ti, tj), tj >= ti, of T tiles.
-__host__ __device__ __forceinline__ int tri_index(int ti, int tj, int T) {
-  return ti * T - (ti * (ti - 1)) / 2 + (tj - ti);
+// The upper triangle in items of 128 beads i by `jt` beads j (a chunk): with
+// T tiles of i and C chunks of j, tile ti meets the chunks from ti * kRefTile /
+// jt on. Items of a tile are numbered one after the other, tile by tile.
+struct RefItems {
+  int P, T, C, per;  // beads, i tiles, j chunks, chunks per tile
+  __host__ __device__ int first(int ti) const { return ti * per; }
+  __host__ __device__ int offset(int ti) const { return ti * C - per * (ti * (ti - 1) / 2); }
+  __host__ __device__ int count() const { return offset(T); }
+};
+// Chunks of 32 beads while items of 128 x 128 would leave the GPU idle (a
+// thread then adds 32 pairs one after the other instead of 128: 1,312 beads
+// took 22.3 us in 66 items, half of them empty CTAs beside them), whole tiles
+// for larger structures, whose items are many anyway.
+constexpr int kRefChunk = 32;
+constexpr int kRefSmallTiles = 48;
+RefItems ref_items(int P, bool chunks = true) {
+  RefItems it;
+  it.P = P;
+  it.T = (P + kRefTile - 1) / kRefTile;
+  const int jt = chunks && it.T <= kRefSmallTiles ? kRefChunk : kRefTile;
+  it.per = kRefTile / jt;
+  it.C = (P + jt - 1) / jt;
+  return it;
 }
 
-__global__ void __launch_bounds__(kRefTile) ref_energy_tiles(
-    const float4* __restrict__ pos, const float4* __restrict__ meta,
-    const float* __restrict__ lj_table, int P, int T, double* __restrict__ partials, RefConsts C) {
-  __shared__ float s_M[400];
-  __shared__ float4 s_jp[kRefTile];
-  __shared__ float4 s_jm[kRefTile];
-  __shared__ double s_red[kRefTile / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < 400; i += kRefTile) s_M[i] = lj_table[i];
-  const float two_third = 1.2599210498948732f;  // 2^(1/3)
-  for (int item = blockIdx.x; item < T * T; item += gridDim.x) {
-    const int ti = item / T, tj = item % T;
-    if (tj < ti) continue;
-    __syncthreads();  // the previous item is done with the j-tile
-    const int j0 = tj * kRefTile;
-    const int jn = min(kRefTile, P - j0);
-    if (tid < jn) {
-      s_jp[tid] = pos[j0 + tid];
-      s_jm[tid] = meta[j0 + tid];
-    }
-    __syncthreads();
-    const int i = ti * kRefTile + tid;
-    float lj = 0.0f, dh = 0.0f;
-    if (i < P) {
-      const float4 pi = pos[i], mi = meta[i];
-      if (pi.w > -2.0f) {  // not a padding bead
-        const bool icrowd = mi.w == -1.0f;
-        const int jstart = (ti == tj) ? tid + 1 : 0;
-        for (int jj = jstart; jj < jn; ++jj) {
-          const float4 pj = s_jp[jj];
-          if (pj.w < 0.0f || pj.w == pi.w) continue;  // padding or same molecule
-          const float4 mj = s_jm[jj];
-          const float r2 = pair_r2(pi, pj, C.box, C.invbox);
-          const float rinv = fast_rsqrt(r2);
-          const float rinv2 = rinv * rinv;
-          if (icrowd || mj.w == -1.0f) {
-            const float i6 = rinv2 * rinv2 * rinv2;
-            if (r2 < C.cutoff2) lj += 46656.0f * i6;  // (6/r)^6
-          } else {
-            int idx = __float2int_rn(20.0f * mi.x + mj.x);
-            idx = min(max(idx, 0), 399);
-            const float eps = C.lambda_ * (s_M[idx] - C.e0);
-            const float sig = (mi.z + mj.z) * 0.5f;
-            const float sig2 = sig * sig;
-            const float s2 = sig2 * rinv2;
-            const float s6 = s2 * s2 * s2;
-            float L = 4.0f * eps * fmaf(-s6, s6, s6);
-            if (eps > 0.0f && r2 < sig2 * two_third) L = 2.0f * eps - L;
-            lj += L;
-            const float r = r2 * rinv;
-            dh += mi.y * mj.y * fast_ex2(r * C.c_xi) * rinv;
-          }
-        }
-      }
-    }
-    double v = (double)lj * (double)C.lj_scale + (double)dh * (double)C.dh_scale;
-    v = warp_sum(v);
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    if (tid == 0) {
-      double t = 0.0;
-      for (int w = 0; w < kRefTile / 32; ++w) t += s_red[w];
-      partials[tri_index(ti, tj, T)] = t;
-    }
-  }
-}
-
-// Fixed-order sum of n partials into *out (one CTA).
-__global__ void ref_energy_sum(const double* __restrict__ partials, int n, double* __restrict__ out,
-                               float* __restrict__ grid_out, int grid_n, float unscale) {
-  __shared__ double s[256];
+// Fixed-order sum of n partials by one CTA; thread 0 has it.
+template <int THREADS>
+__device__ double sum_partials(const volatile double* partials, int n, double* s) {
   double v = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) v += partials[i];
+  for (int i = threadIdx.x; i < n; i += THREADS) v += partials[i];
   s[threadIdx.x] = v;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+  for (int w = THREADS / 2; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0 && out) *out = s[0];
-  if (grid_out) {
-    // the reference's per-block layout: the host sums it and scales by KBT_CF
-    for (int i = threadIdx.x; i < grid_n; i += blockDim.x)
-      grid_out[i] = (i == 0) ? (float)(s[0] * (double)unscale) : 0.0f;
+  return s[0];
+}
+
+// Where the total goes: *out, and the reference's per-block layout (the host
+// sums it and scales by KBT_CF).
+struct RefTotal {
+  double* out;
+  float* grid_out;
+  int grid_n;
+  float unscale;
+};
+__device__ void put_total(double total, const RefTotal& R) {
+  if (threadIdx.x == 0 && R.out) *R.out = total;
+  if (R.grid_out)
+    for (int i = threadIdx.x; i < R.grid_n; i += blockDim.x)
+      R.grid_out[i] = (i == 0) ? (float)(total * (double)R.unscale) : 0.0f;
+}
+
+// One item per CTA (chunk blockIdx.x, tile blockIdx.y). With `done` the last CTA
+// to finish adds the partials, in a fixed order, and sets the counter back.
+template <int JT>
+__global__ void __launch_bounds__(kRefTile) ref_energy_tiles(
+    const float4* __restrict__ pos, const float4* __restrict__ meta,
+    const float* __restrict__ lj_table, RefItems it, double* __restrict__ partials, RefConsts C,
+    unsigned* __restrict__ done, RefTotal total) {
+  const int ti = blockIdx.y, c = blockIdx.x;
+  if (c < it.first(ti)) return;
+  __shared__ float s_eps[400];
+  __shared__ float4 s_jp[JT], s_jm[JT];
+  __shared__ double s_red[kRefTile];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < 400; i += kRefTile) s_eps[i] = C.lambda_ * (lj_table[i] - C.e0);
+  const int j0 = c * JT, jn = min(JT, it.P - j0);
+  if (tid < JT) {  // places past the last bead hold padding
+    s_jp[tid] = tid < jn ? pos[j0 + tid] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+    s_jm[tid] = tid < jn ? meta[j0 + tid] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
+  const int i = ti * kRefTile + tid;
+  const bool valid = i < it.P;
+  const float4 pi = valid ? pos[i] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+  const float4 mi = valid ? meta[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const bool counts = pi.w > -2.0f;  // not a padding bead
+  const bool icrowd = mi.w == -1.0f;
+  const float row = 20.0f * mi.x;
+  const float two_third = 1.2599210498948732f;  // 2^(1/3)
+  __syncthreads();
+  float lj = 0.0f, dh = 0.0f;
+#pragma unroll 4
+  for (int jj = 0; jj < JT; ++jj) {
+    const float4 pj = s_jp[jj], mj = s_jm[jj];
+    // padding, the same molecule, or (diagonal) an earlier bead
+    const bool use = counts && j0 + jj > i && !(pj.w < 0.0f) && pj.w != pi.w;
+    const float r2 = pair_r2(pi, pj, C.box, C.invbox);
+    const float rinv = fast_rsqrt(r2);
+    const float rinv2 = rinv * rinv;
+    if (icrowd || mj.w == -1.0f) {
+      const float i6 = rinv2 * rinv2 * rinv2;
+      if (use && r2 < C.cutoff2) lj += 46656.0f * i6;  // (6/r)^6
+    } else if (use) {
+      // rint of the index, as an integer, without a conversion
+      int idx = __float_as_int(__fadd_rn(__fadd_rn(row, mj.x), 12582912.0f)) - 0x4b400000;
+      idx = min(max(idx, 0), 399);
+      const float eps = s_eps[idx];
+      const float sig = (mi.z + mj.z) * 0.5f;
+      const float sig2 = sig * sig;
+      const float s2 = sig2 * rinv2;
+      const float s6 = s2 * s2 * s2;
+      float L = 4.0f * eps * fmaf(-s6, s6, s6);
+      if (eps > 0.0f && r2 < sig2 * two_third) L = 2.0f * eps - L;
+      lj += L;
+      const float r = r2 * rinv;
+      dh += mi.y * mj.y * fast_ex2(r * C.c_xi) * rinv;
+    }
+  }
+  double v = (double)lj * (double)C.lj_scale + (double)dh * (double)C.dh_scale;
+  v = warp_sum(v);
+  if (lane == 0) s_red[warp] = v;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < kRefTile / 32; ++w) t += s_red[w];
+    partials[it.offset(ti) + c - it.first(ti)] = t;
+    if (done) {
+      __threadfence();
+      s_last = atomicAdd(done, 1u) == (unsigned)it.count() - 1u;
+    }
+  }
+  if (!done) return;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const double sum = sum_partials<kRefTile>(partials, it.count(), s_red);
+  put_total(sum, total);
+  if (tid == 0) *done = 0u;
+}
+
+// Fixed-order sum of n partials (one CTA), for the call whose calls may overlap
+// and so cannot share a counter.
+__global__ void ref_energy_sum(const double* __restrict__ partials, int n, RefTotal total) {
+  __shared__ double s[256];
+  put_total(sum_partials<256>(partials, n, s), total);
+}
+
+// Launch the items; `done` (may be null): the last CTA adds the partials.
+cudaError_t launch_ref_items(const float4* pos, const float4* meta, const float* table,
+                             const RefItems& it, double* partials, const RefConsts& C,
+                             unsigned* done, const RefTotal& total, cudaStream_t stream) {
+  const dim3 grid(it.C, it.T);
+  if (it.per == 1)
+    ref_energy_tiles<kRefTile><<<grid, kRefTile, 0, stream>>>(pos, meta, table, it, partials, C, done, total);
+  else
+    ref_energy_tiles<kRefChunk><<<grid, kRefTile, 0, stream>>>(pos, meta, table, it, partials, C, done, total);
+  return cudaGetLastError();
 }
 
 __global__ void rotate_molecule_kernel(float4* pos, const int* start, const int* length,
@@ -247,7 +306,9 @@ double* stream_scratch(cudaStream_t stream, size_t n, std::unique_lock<std::mute
       slot->cap = 0;
     }
     const size_t cap = std::max<size_t>(n, 4096);
-    if (cudaMalloc(&slot->ptr, cap * sizeof(double)) != cudaSuccess) {
+    if (cudaMalloc(&slot->ptr, cap * sizeof(double)) != cudaSuccess ||
+        cudaMemsetAsync(slot->ptr, 0, sizeof(double), stream) != cudaSuccess) {
+      cudaFree(slot->ptr);
       slot->ptr = nullptr;
       return nullptr;
     }
@@ -284,28 +345,21 @@ bool energy_args_ok(const float4* pos, const float4* meta, const float* table, i
   return true;
 }
 
-// Enqueue the energy of P beads on `stream`: partials in scratch[0..n),
-// total in scratch[n]; optionally the reference's per-block grid.
+// Doubles of scratch for an energy call: the counter of finished items (zero
+// between calls, which take turns on their stream), the total, the partials.
+size_t ref_scratch(int P) { return (size_t)ref_items(P).count() + 2; }
+
+// Enqueue the energy of P beads on `stream`; the total goes to scratch[1] and,
+// optionally, to the reference's per-block grid.
 int enqueue_energy(const float4* pos, const float4* meta, const float* table, int P,
                    double* scratch, float* grid_out, int grid_n, cudaStream_t stream) {
-  const int T = (P + kRefTile - 1) / kRefTile;
-  const int n = T * (T + 1) / 2;
-  float unscale = 1.0f;
-  const RefConsts C = make_consts(&unscale);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::min(T * T, sms * 8);
-  ref_energy_tiles<<<grid, kRefTile, 0, stream>>>(pos, meta, table, P, T, scratch, C);
-  cudaError_t e = cudaGetLastError();
+  RefTotal total{scratch + 1, grid_out, grid_n, 1.0f};
+  const RefConsts C = make_consts(&total.unscale);
+  const cudaError_t e =
+      launch_ref_items(pos, meta, table, ref_items(P), scratch + 2, C,
+                       reinterpret_cast<unsigned*>(scratch), total, stream);
   if (e != cudaSuccess) {
     set_status(REMC_ERR_CUDA, "energy kernel launch", e);
-    return REMC_ERR_CUDA;
-  }
-  ref_energy_sum<<<1, 256, 0, stream>>>(scratch, n, scratch + n, grid_out, grid_n, unscale);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_status(REMC_ERR_CUDA, "energy sum launch", e);
     return REMC_ERR_CUDA;
   }
   return REMC_OK;
@@ -402,19 +456,17 @@ void CUDA_EonDevice(float4* pos, float4* meta, int* residueCount, int* moleculeP
     return;
   }
   if (!energy_args_ok(pos, meta, table, datasetSize)) return;
-  const int T = (datasetSize + kRefTile - 1) / kRefTile;
-  const size_t n = (size_t)T * (T + 1) / 2;
   // the reference's synchronous path runs on the legacy default stream; the
   // result copy is made under the scratch lock, before another host thread
   // can queue its energy on the same buffer
   std::unique_lock<std::mutex> lock;
-  double* scratch = stream_scratch(0, n + 1, lock);
+  double* scratch = stream_scratch(0, ref_scratch(datasetSize), lock);
   if (!scratch) {
     set_status(REMC_ERR_NOMEM, "scratch allocation failed");
     return;
   }
   if (enqueue_energy(pos, meta, table, datasetSize, scratch, nullptr, 0, 0) != REMC_OK) return;
-  cudaError_t e = cudaMemcpy(result, scratch + n, sizeof(double), cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemcpy(result, scratch + 1, sizeof(double), cudaMemcpyDeviceToHost);
   set_status(e == cudaSuccess ? REMC_OK : REMC_ERR_CUDA, "result copy", e);
 }
 
@@ -433,13 +485,11 @@ void CUDA_EonDevice_async(float4* pos, float4* meta, int* residueCount, int* mol
     return;
   }
   if (!energy_args_ok(pos, meta, table, datasetSize)) return;
-  const int T = (datasetSize + kRefTile - 1) / kRefTile;
-  const size_t n = (size_t)T * (T + 1) / 2;
   // the stream's own scratch: energies queued on other streams run
   // concurrently on other buffers, and the next call on this stream reuses
   // this one only after this call's kernels, in stream order
   std::unique_lock<std::mutex> lock;
-  double* scratch = stream_scratch(stream, n + 1, lock);
+  double* scratch = stream_scratch(stream, ref_scratch(datasetSize), lock);
   if (!scratch) {
     set_status(REMC_ERR_NOMEM, "scratch allocation failed");
     return;
@@ -515,9 +565,10 @@ int CUDA_EonDevice_noalloc(const float4* pos, const float4* meta, const float* L
     return REMC_ERR_INVALID;
   }
   if (!energy_args_ok(pos, meta, table, datasetSize)) return g_status;
-  const int T = (datasetSize + kRefTile - 1) / kRefTile;
-  const long long n = (long long)T * (T + 1) / 2;
-  if (n > kNoAllocMaxItems) {
+  // chunks while their items fit the fixed scratch
+  RefItems it = ref_items(datasetSize);
+  if (it.count() > kNoAllocMaxItems) it = ref_items(datasetSize, false);
+  if ((long long)it.T * (it.T + 1) / 2 > kNoAllocMaxItems) {
     char buf[160];
     snprintf(buf, sizeof(buf),
              "datasetSize %d exceeds the allocation-free limit of %d beads (%d tile pairs)",
@@ -548,16 +599,12 @@ int CUDA_EonDevice_noalloc(const float4* pos, const float4* meta, const float* L
   }
   // every item writes its partial before the sum reads it: no clearing needed
   const RefConsts C = make_consts();
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::min(T * T, sms * 8);
-  ref_energy_tiles<<<grid, kRefTile, 0, stream>>>(pos, meta, table, datasetSize, T, scratch, C);
-  e = cudaGetLastError();
+  e = launch_ref_items(pos, meta, table, it, scratch, C, nullptr, RefTotal{}, stream);
   if (e != cudaSuccess) {
     set_status(REMC_ERR_CUDA, "energy kernel launch", e);
     return REMC_ERR_CUDA;
   }
-  ref_energy_sum<<<1, 256, 0, stream>>>(scratch, (int)n, d_result, nullptr, 0, 1.0f);
+  ref_energy_sum<<<1, 256, 0, stream>>>(scratch, it.count(), RefTotal{d_result, nullptr, 0, 1.0f});
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_status(REMC_ERR_CUDA, "energy sum launch", e);
