@@ -185,39 +185,147 @@ __global__ void __launch_bounds__(256) rank_kernel(const long long* __restrict__
 // Host layout (3 floats per bead and molecule) <-> device layout (float4 with
 // the bead meta word), converted on the device so that uploads and downloads
 // are plain copies of the caller's buffers.
-__global__ void state_check_kernel(const float* __restrict__ pos3, const float* __restrict__ rel3,
-                                   const float* __restrict__ cen3, const int* __restrict__ info,
-                                   long long nb, long long nm,
-                                   unsigned long long* __restrict__ bad) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nb; i += stride) {
-    const float* p = pos3 + 3 * i;
-    const float* r = rel3 + 3 * i;
-    bool fin = true;
-    for (int k = 0; k < 3; ++k) fin = fin && isfinite(p[k]) && isfinite(r[k]);
-    if (!fin) atomicMin(&bad[0], (unsigned long long)i);
-    if ((info[i] & (int)0x80000000u) && (r[0] != 0.0f || r[1] != 0.0f || r[2] != 0.0f))
-      atomicMin(&bad[1], (unsigned long long)i);
+//
+// state_scan_kernel reads the staged state once: it checks every coordinate
+// and gathers what decides the fold flags. state_pack_kernel runs only after
+// the host has seen that nothing is wrong, so a refused upload changes nothing.
+//
+// May the sweep fold the minimum image of a system? A bead the sweep has not
+// moved is where it was uploaded; a moved molecule has its centre in [0, L)
+// (translations wrap it, rotations leave it) and each bead within R of it (a
+// rotation of rel keeps |rel|), R the largest |rel| over all instances. So on
+// each axis every bead lies in [min(p_min, -R), max(p_max, L + R)], and no two
+// are further apart than that interval is long. fold_image2 needs less than
+// 1.5 L; the test keeps a margin (1.01 R, 1.49 L) for the rounding of repeated
+// rotations. Each CTA leaves its largest |rel|^2 and bead extent in column
+// `cta` of part (rows R^2, -p_min xyz, p_max xyz, all combined by max), and the
+// last CTA to finish combines a system's columns.
+struct ScanResult {
+  unsigned long long bad[3];  // first bead not finite, bead off its centre, centre not finite
+  unsigned done;              // CTAs that have finished
+  unsigned pad;
+};
+constexpr int kScanBeads = 1024;  // beads of an instance per CTA
+
+// what state_scan_kernel leaves where the host reads it
+struct ScanReport {
+  unsigned long long bad[3];
+  int fold[1];  // per system
+};
+
+__device__ __forceinline__ float warp_max(float v) {
+  for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+  return v;
+}
+
+__global__ void __launch_bounds__(256) state_scan_kernel(
+    const SysDev* __restrict__ sys, const int* __restrict__ inst_sys, int n_sys,
+    const float* __restrict__ pos3, const float* __restrict__ rel3, const float* __restrict__ cen3,
+    const int* __restrict__ info, float* __restrict__ part, ScanResult* __restrict__ res,
+    int* __restrict__ fold, ScanReport* __restrict__ report) {
+  __shared__ float s_v[8][8];
+  __shared__ bool s_last;
+  const int inst = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n_cta = gridDim.x * gridDim.y;
+  const float lowest = -3.0e38f;
+  {
+    const SysDev S = sys[inst_sys[inst]];
+    const int slot = inst - S.inst0;
+    const long long b0 = S.bead_base + (long long)slot * S.n_beads;
+    const long long m0 = S.mol_base + (long long)slot * S.n_mol;
+    const int from = blockIdx.y * kScanBeads, to = min(S.n_beads, from + kScanBeads);
+    float v[7] = {0.0f, lowest, lowest, lowest, lowest, lowest, lowest};
+    for (int k = from + tid; k < to; k += blockDim.x) {
+      const long long i = b0 + k;
+      const float px = pos3[3 * i], py = pos3[3 * i + 1], pz = pos3[3 * i + 2];
+      const float rx = rel3[3 * i], ry = rel3[3 * i + 1], rz = rel3[3 * i + 2];
+      if (!(isfinite(px) && isfinite(py) && isfinite(pz) && isfinite(rx) && isfinite(ry) && isfinite(rz)))
+        atomicMin(&res->bad[0], (unsigned long long)i);
+      if (info[i] < 0 && (rx != 0.0f || ry != 0.0f || rz != 0.0f))
+        atomicMin(&res->bad[1], (unsigned long long)i);
+      v[0] = fmaxf(v[0], fmaf(rx, rx, fmaf(ry, ry, rz * rz)));
+      v[1] = fmaxf(v[1], -px);
+      v[2] = fmaxf(v[2], -py);
+      v[3] = fmaxf(v[3], -pz);
+      v[4] = fmaxf(v[4], px);
+      v[5] = fmaxf(v[5], py);
+      v[6] = fmaxf(v[6], pz);
+    }
+    for (int m = blockIdx.y * kScanBeads + tid; m < min(S.n_mol, from + kScanBeads); m += blockDim.x) {
+      const float* c = cen3 + 3 * (m0 + m);
+      if (!(isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2])))
+        atomicMin(&res->bad[2], (unsigned long long)(m0 + m));
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      v[k] = warp_max(v[k]);
+      if (lane == 0) s_v[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (tid < 7) {
+      float w = s_v[tid][0];
+      for (int q = 1; q < 8; ++q) w = fmaxf(w, s_v[tid][q]);
+      part[(size_t)tid * n_cta + inst * gridDim.y + blockIdx.y] = w;
+      __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&res->done, 1u) == (unsigned)n_cta - 2u;  // counts from ~0
+    __syncthreads();
+    if (!s_last) return;
   }
-  for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < nm; m += stride) {
-    const float* c = cen3 + 3 * m;
-    if (!(isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2])))
-      atomicMin(&bad[2], (unsigned long long)m);
+  __threadfence();
+  // the last CTA: systems by warp, or all warps on one system's columns at a time
+  const bool together = n_sys < 8;
+  const int step = together ? 1 : 8;
+  const volatile float* columns = part;
+  for (int q = together ? 0 : warp; q < n_sys; q += step) {
+    const SysDev S = sys[q];
+    const int a = S.inst0 * (int)gridDim.y, e = (S.inst0 + S.n_rep) * (int)gridDim.y;
+    float w[7] = {0.0f, lowest, lowest, lowest, lowest, lowest, lowest};
+    for (int i = a + (together ? tid : lane); i < e; i += together ? 256 : 32)
+#pragma unroll
+      for (int k = 0; k < 7; ++k) w[k] = fmaxf(w[k], columns[(size_t)k * n_cta + i]);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) w[k] = warp_max(w[k]);
+    if (together) {
+      __syncthreads();
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 7; ++k) s_v[k][warp] = w[k];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 7; ++k)
+        for (int p = 0; p < 8; ++p) w[k] = fmaxf(w[k], s_v[k][p]);
+    }
+    if (lane == 0 && (!together || warp == 0)) {
+      const float R = 1.01f * sqrtf(w[0]), lim = 1.49f * S.box;
+      bool ok = true;
+      for (int c = 0; c < 3; ++c)  // max(p_max, L + R) - min(p_min, -R)
+        ok = ok && fmaxf(w[4 + c], S.box + R) + fmaxf(w[1 + c], R) <= lim;
+      fold[q] = ok ? 1 : 0;
+      report->fold[q] = ok ? 1 : 0;
+    }
   }
+  if (tid < 3) report->bad[tid] = *(volatile unsigned long long*)&res->bad[tid];
 }
 
 __global__ void state_pack_kernel(const float* __restrict__ pos3, const float* __restrict__ rel3,
-                                  const float* __restrict__ cen3, const int* __restrict__ info,
-                                  long long nb, long long nm, float4* __restrict__ pos,
-                                  float4* __restrict__ rel, float4* __restrict__ cen) {
+                                  const float* __restrict__ cen3, const double2* __restrict__ quat4,
+                                  const int* __restrict__ info, const int* __restrict__ fold,
+                                  long long nb, long long nm, int n_sys, float4* __restrict__ pos,
+                                  float4* __restrict__ rel, float4* __restrict__ cen,
+                                  double2* __restrict__ quat, SysDev* __restrict__ sys) {
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nb; i += stride) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = first; i < nb; i += stride) {
     pos[i] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2],
                          __int_as_float(info[i] & 0x7fffffff));
     rel[i] = make_float4(rel3[3 * i], rel3[3 * i + 1], rel3[3 * i + 2], 0.0f);
   }
-  for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < nm; m += stride)
+  for (long long m = first; m < nm; m += stride)
     cen[m] = make_float4(cen3[3 * m], cen3[3 * m + 1], cen3[3 * m + 2], 0.0f);
+  for (long long k = first; k < 2 * nm; k += stride) quat[k] = quat4[k];
+  for (long long q = first; q < n_sys; q += stride) sys[q].fold_mi = fold[q];
 }
 
 __global__ void state_unpack_kernel(const float4* __restrict__ pos, const float4* __restrict__ rel,
@@ -239,78 +347,6 @@ __global__ void state_unpack_kernel(const float4* __restrict__ pos, const float4
     cen3[3 * m] = c.x;
     cen3[3 * m + 1] = c.y;
     cen3[3 * m + 2] = c.z;
-  }
-}
-
-// May the sweep fold the minimum image of a system? A bead the sweep has not
-// moved is where it was uploaded; a moved molecule has its centre in [0, L)
-// (translations wrap it, rotations leave it) and each bead within R of it (a
-// rotation of rel keeps |rel|), R the largest |rel| over all instances. So on
-// each axis every bead lies in [min(p_min, -R), max(p_max, L + R)], and no two
-// are further apart than that interval is long. fold_image2 needs less than
-// 1.5 L; the test keeps a margin (1.01 R, 1.49 L) for the rounding of repeated
-// rotations. fold_part_kernel: one CTA per instance, its largest |rel|^2 and
-// bead extent (part[inst][0..6]: R^2, -p_min xyz, p_max xyz, all combined by
-// max); fold_flag_kernel: one CTA per system combines its instances.
-__global__ void fold_part_kernel(const SysDev* __restrict__ sys, const int* __restrict__ inst_sys,
-                                 const float4* __restrict__ pos, const float4* __restrict__ rel,
-                                 float* __restrict__ part) {
-  __shared__ float s_v[7][32];
-  const int inst = blockIdx.x;
-  const SysDev S = sys[inst_sys[inst]];
-  const size_t base = S.bead_base + (size_t)(inst - S.inst0) * S.n_beads;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float lowest = -3.0e38f;
-  float v[7] = {0.0f, lowest, lowest, lowest, lowest, lowest, lowest};
-  for (int i = tid; i < S.n_beads; i += blockDim.x) {
-    const float4 q = rel[base + i], p = pos[base + i];
-    v[0] = fmaxf(v[0], fmaf(q.x, q.x, fmaf(q.y, q.y, q.z * q.z)));
-    v[1] = fmaxf(v[1], -p.x);
-    v[2] = fmaxf(v[2], -p.y);
-    v[3] = fmaxf(v[3], -p.z);
-    v[4] = fmaxf(v[4], p.x);
-    v[5] = fmaxf(v[5], p.y);
-    v[6] = fmaxf(v[6], p.z);
-  }
-#pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    for (int off = 16; off > 0; off >>= 1) v[k] = fmaxf(v[k], __shfl_down_sync(0xffffffffu, v[k], off));
-    if (lane == 0) s_v[k][warp] = v[k];
-  }
-  __syncthreads();
-  if (tid < 7) {
-    float w = s_v[tid][0];
-    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) w = fmaxf(w, s_v[tid][q]);
-    part[(size_t)inst * 8 + tid] = w;
-  }
-}
-
-__global__ void fold_flag_kernel(SysDev* __restrict__ sys, const float* __restrict__ part) {
-  __shared__ float s_v[7][32];
-  const SysDev S = sys[blockIdx.x];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float lowest = -3.0e38f;
-  float v[7] = {0.0f, lowest, lowest, lowest, lowest, lowest, lowest};
-  for (int i = tid; i < S.n_rep; i += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 7; ++k) v[k] = fmaxf(v[k], part[(size_t)(S.inst0 + i) * 8 + k]);
-#pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    for (int off = 16; off > 0; off >>= 1) v[k] = fmaxf(v[k], __shfl_down_sync(0xffffffffu, v[k], off));
-    if (lane == 0) s_v[k][warp] = v[k];
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float w[7];
-    for (int k = 0; k < 7; ++k) {
-      w[k] = s_v[k][0];
-      for (int q = 1; q < (int)(blockDim.x >> 5); ++q) w[k] = fmaxf(w[k], s_v[k][q]);
-    }
-    const float R = 1.01f * sqrtf(w[0]), lim = 1.49f * S.box;
-    bool ok = true;
-    for (int a = 0; a < 3; ++a)  // max(p_max, L + R) - min(p_min, -R)
-      ok = ok && fmaxf(w[4 + a], S.box + R) + fmaxf(w[1 + a], R) <= lim;
-    sys[blockIdx.x].fold_mi = ok ? 1 : 0;
   }
 }
 
@@ -524,7 +560,7 @@ __global__ void __launch_bounds__(kTile) energy_tile_kernel(
     // the previous item (its tile buffer, coordinate copy and partials)
     if (__syncthreads_or(!ok)) {  // the copy never landed: report and stop
       if (tid == 0) {
-        atomicOr(err, 1);
+        *(volatile int*)err = 1;
         // the copy given up on still writes this CTA's shared memory (the
         // next one is not issued yet): wait for it again, bounded, before
         // the CTA leaves; it can leave with the copy in flight only if this
@@ -608,14 +644,17 @@ __global__ void wait_probe_kernel(int* __restrict__ err, int polls) {
   if (threadIdx.x == 0) mbar_init(&s_bar, 1);
   __syncthreads();
   const bool ok = mbar_wait(&s_bar, 0u, polls);
-  if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicOr(err, 1);
+  if (__syncthreads_or(!ok) && threadIdx.x == 0) *(volatile int*)err = 1;
 }
 
-// Per-instance fixed-order sum of the tile partials.
+// Per-instance fixed-order sum of the tile partials, also to `host` (memory the
+// host reads; may be null). Sets the tile kernel's work queue back to zero.
 __global__ void energy_reduce_kernel(const int* __restrict__ item_off, int n_inst,
                                      const double* __restrict__ scratch,
                                      const double* __restrict__ scratch_cc,
-                                     double* __restrict__ energy, double* __restrict__ ecc) {
+                                     double* __restrict__ energy, double* __restrict__ ecc,
+                                     double* __restrict__ host, int* __restrict__ queue) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0;
   const int inst = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (inst >= n_inst) return;
@@ -630,6 +669,7 @@ __global__ void energy_reduce_kernel(const int* __restrict__ item_off, int n_ins
   if (lane == 0) {
     energy[inst] = v;
     ecc[inst] = c;
+    if (host) host[inst] = v;
   }
 }
 
@@ -1189,7 +1229,15 @@ struct remc_handle {
   int sweep_cluster_slots = 0;  // clusters of that size the GPU holds at once
   int beads_in_smem = 1; // beads resident in shared memory (else updated in place in global)
   float4* d_sweep_scratch = nullptr;  // what a sweep CTA does not hold in shared memory
-  float* d_fold_part = nullptr;       // per instance: the fold test's partial extents [8]
+  float* d_scan_part = nullptr;       // the upload scan's partial extents [7][CTA]
+  ScanResult* d_scan = nullptr;       // its counters, then the systems' fold flags
+  int scan_rows = 1;                  // its CTAs per instance
+  // pinned host memory that kernels write: the error word of bounded waits, the
+  // upload scan's report, energies
+  unsigned char* h_pin = nullptr;
+  int* pin_err = nullptr;
+  ScanReport* pin_scan = nullptr;
+  double* pin_energy = nullptr;
   size_t sweep_scratch_cap = 0;       // float4 entries
   int max_dyn_smem = 0;
   int config_gen = 0;  // bumped when the sweep schedule changes
@@ -1225,8 +1273,6 @@ struct remc_handle {
   int* d_bead_info = nullptr;  // per bead per instance: meta word | (one-bead molecule << 31)
   float* d_stage = nullptr;    // host-layout staging: pos[3n], rel[3n], centre[3m]
   double* d_stage_q = nullptr; // quaternions [4m]
-  unsigned long long* d_bad = nullptr;  // first invalid bead / one-bead offset / molecule
-  int* d_err = nullptr;        // set by a kernel whose bounded wait gave up
   int sweep_threads = 128;  // virtual threads per CTA (the schedule's threads per replica)
   int sweep_block = 256;    // threads per CTA
   SweepShape sweep_shape{};
@@ -1268,10 +1314,11 @@ void free_all(remc_handle* h) {
                   h->d_mft,
                   h->d_ctrl,     h->d_items_by_cost, h->d_energy_queue,
                   h->d_item_off,   h->d_scratch,    h->d_newpos,
-                  h->d_dE,       h->d_bead_info, h->d_stage,      h->d_stage_q,    h->d_bad,
-                  h->d_err,      h->d_sweep_scratch, h->d_fold_part};
+                  h->d_dE,       h->d_bead_info, h->d_stage,      h->d_stage_q,
+                  h->d_sweep_scratch, h->d_scan_part, h->d_scan};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
@@ -1335,11 +1382,9 @@ struct NvtxRange {
 
 // Report (and clear) the error word a kernel sets when a bounded wait gives up.
 int check_device_error(remc_handle* h) {
-  int e = 0;
-  REMC_CUDA_TRY(cudaMemcpyAsync(&e, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  if (e) {
-    REMC_CUDA_TRY(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
+  if (*(volatile int*)h->pin_err) {
+    *(volatile int*)h->pin_err = 0;
     return set_error(REMC_ERR_TIMEOUT, "a device-side wait for a bulk copy gave up");
   }
   return REMC_OK;
@@ -1373,6 +1418,20 @@ SweepFn sweep_fn(const remc_handle* h, bool cluster, bool global_beads) {
   const bool cut = h->params.crowder_cutoff > 0.0f, fold = h->all_fold;
   return h->params.crowder_mode ? sweep_fn_wall(cut, fold, cluster, global_beads)
                                 : sweep_fn_reference(cut, fold, cluster, global_beads);
+}
+
+// Let the sweep kernels of a layout (folded or not) use all shared memory.
+int allow_smem(const remc_handle* h, bool cluster, bool global_beads) {
+  const bool cut = h->params.crowder_cutoff > 0.0f;
+  for (int fold = 0; fold < 2; ++fold) {
+    const SweepFn f = h->params.crowder_mode ? sweep_fn_wall(cut, fold, cluster, global_beads)
+                                             : sweep_fn_reference(cut, fold, cluster, global_beads);
+    const cudaError_t e =
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_dyn_smem);
+    if (e != cudaSuccess)
+      return set_error(REMC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  return REMC_OK;
 }
 
 // Shared-memory shape of a sweep launch, without the parts it can do without.
@@ -1421,6 +1480,7 @@ constexpr double kSpreadPairs = 4096.0;
 // Add to a shape what fits in shared memory beside it without taking CTAs off
 // the SM, and find how many CTAs an SM, and clusters the GPU, hold.
 int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* clusters) {
+  if (allow_smem(h, shape.csize > 1, !shape.beads_in_smem)) return REMC_ERR_CUDA;
   const SweepFn fn = sweep_fn(h, shape.csize > 1, !shape.beads_in_smem);
   auto resident = [&](const SweepShape& p) {
     const size_t smem = SweepSmem::make(p).total;
@@ -1807,30 +1867,14 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   int max_smem = 0;
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
   cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
-  SweepFn kSweeps[32];
-  for (int k = 0; k < 16; ++k) {
-    kSweeps[k] = sweep_fn_wall(k & 1, k & 2, k & 4, k & 8);
-    kSweeps[16 + k] = sweep_fn_reference(k & 1, k & 2, k & 4, k & 8);
+  cudaFuncAttributes fattr;  // the sweep kernels have the same static shared memory
+  e = cudaFuncGetAttributes(&fattr, sweep_fn(h, false, false));
+  if (e != cudaSuccess) {
+    delete h;
+    return set_error(REMC_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
   }
-  int static_smem = 0;
-  for (SweepFn f : kSweeps) {
-    cudaFuncAttributes fattr;
-    e = cudaFuncGetAttributes(&fattr, f);
-    if (e != cudaSuccess) {
-      delete h;
-      return set_error(REMC_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
-    }
-    static_smem = std::max(static_smem, (int)fattr.sharedSizeBytes);
-  }
-  const int max_dyn = max_smem - static_smem;
+  const int max_dyn = max_smem - (int)fattr.sharedSizeBytes;
   h->max_dyn_smem = max_dyn;
-  for (SweepFn f : kSweeps) {
-    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
-    if (e != cudaSuccess) {
-      delete h;
-      return set_error(REMC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
-  }
   // default schedule (the autotuner may replace it): molecule data in shared
   // memory when it fits, more threads per replica for larger systems, and the
   // beads left in global memory for systems too large for shared memory
@@ -1907,8 +1951,6 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   if (!rc) rc = dev_alloc(&h->d_bead_info, h->total_beads);
   if (!rc) rc = dev_alloc(&h->d_stage, 6 * h->total_beads + 3 * h->total_mols);
   if (!rc) rc = dev_alloc(&h->d_stage_q, 4 * h->total_mols);
-  if (!rc) rc = dev_alloc(&h->d_bad, 3);
-  if (!rc) rc = dev_alloc(&h->d_err, 1);
   if (!rc) rc = dev_alloc(&h->d_rel, h->total_beads);
   if (!rc) rc = dev_alloc(&h->d_centre, h->total_mols);
   if (!rc) rc = dev_alloc(&h->d_quat, 4 * h->total_mols);
@@ -1942,7 +1984,23 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   if (!rc) rc = dev_alloc(&h->d_sample_cursor, 4);
   if (!rc) rc = dev_alloc(&h->d_newpos, h->lmax);
   if (!rc) rc = dev_alloc(&h->d_dE, 1);
-  if (!rc) rc = dev_alloc(&h->d_fold_part, (size_t)h->n_inst * 8);
+  h->scan_rows = (std::max(h->nmax, h->mmax) + kScanBeads - 1) / kScanBeads;
+  if (!rc) rc = dev_alloc(&h->d_scan_part, (size_t)h->n_inst * h->scan_rows * 7);
+  if (!rc)
+    rc = dev_alloc((unsigned char**)&h->d_scan, sizeof(ScanResult) + sizeof(int) * h->n_sys);
+  if (!rc) {
+    const size_t o_scan = 16, o_energy = (o_scan + sizeof(ScanReport) + sizeof(int) * h->n_sys + 15) & ~(size_t)15;
+    if (cudaHostAlloc((void**)&h->h_pin, o_energy + sizeof(double) * h->n_inst, cudaHostAllocMapped) !=
+        cudaSuccess) {
+      h->h_pin = nullptr;
+      rc = set_error(REMC_ERR_NOMEM, "pinned host memory");
+    } else {
+      h->pin_err = reinterpret_cast<int*>(h->h_pin);
+      h->pin_scan = reinterpret_cast<ScanReport*>(h->h_pin + o_scan);
+      h->pin_energy = reinterpret_cast<double*>(h->h_pin + o_energy);
+      *h->pin_err = 0;
+    }
+  }
   auto up = [&](void* dst, const void* src, size_t bytes) {
     if (rc) return;
     cudaError_t ee = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
@@ -1986,7 +2044,7 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
     cudaMemsetAsync(h->d_ex_acc, 0, sizeof(int) * h->n_sys, h->stream);
     cudaMemsetAsync(h->d_energy, 0, sizeof(double) * h->n_inst, h->stream);
     cudaMemsetAsync(h->d_ecc, 0, sizeof(double) * h->n_inst, h->stream);
-    cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
+    cudaMemsetAsync(h->d_energy_queue, 0, sizeof(int), h->stream);
     cudaMemsetAsync(h->d_n_samples, 0, sizeof(int) * h->n_inst, h->stream);
     cudaMemsetAsync(h->d_n_bound, 0, sizeof(int) * h->n_inst, h->stream);
     cudaMemsetAsync(h->d_sample_cursor, 0, sizeof(unsigned) * 4, h->stream);
@@ -2017,6 +2075,9 @@ int remc_set_params(remc_handle* h, const remc_params* p) {
     return set_error(REMC_ERR_INVALID, "bad parameters");
   h->params = *p;
   h->config_gen++;  // a captured graph holds the old constants and kernel
+  if (allow_smem(h, h->sweep_shape.csize > 1, !h->beads_in_smem) ||
+      allow_smem(h, false, !h->beads_in_smem))
+    return REMC_ERR_CUDA;
   if (h->tables_set) return build_tables(h);
   return REMC_OK;
 }
@@ -2050,15 +2111,17 @@ int remc_upload_state(remc_handle* h, const float* pos, const float* rel, const 
                                 h->stream));
   REMC_CUDA_TRY(cudaMemcpyAsync(h->d_stage_q, quat, sizeof(double) * 4 * nm,
                                 cudaMemcpyHostToDevice, h->stream));
-  REMC_CUDA_TRY(cudaMemsetAsync(h->d_bad, 0x7f, sizeof(unsigned long long) * 3, h->stream));
-  const int grid = h->num_sms * 4;
-  state_check_kernel<<<grid, 256, 0, h->stream>>>(sp, sr, sc, h->d_bead_info, (long long)nb,
-                                                  (long long)nm, h->d_bad);
+  // all ones: the counters hold indexes by minimum, and count up from -1
+  REMC_CUDA_TRY(cudaMemsetAsync(h->d_scan, 0xff, sizeof(ScanResult), h->stream));
+  int* const fold = reinterpret_cast<int*>(h->d_scan + 1);
+  state_scan_kernel<<<dim3(h->n_inst, h->scan_rows), 256, 0, h->stream>>>(
+      h->d_sys, h->d_inst_sys, h->n_sys, sp, sr, sc, h->d_bead_info, h->d_scan_part, h->d_scan, fold,
+      h->pin_scan);
   REMC_CUDA_TRY(cudaGetLastError());
-  unsigned long long bad[3];
-  REMC_CUDA_TRY(cudaMemcpyAsync(bad, h->d_bad, sizeof(bad), cudaMemcpyDeviceToHost, h->stream));
   REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  const unsigned long long none = 0x7f7f7f7f7f7f7f7full;
+  unsigned long long bad[3];
+  for (int k = 0; k < 3; ++k) bad[k] = ((volatile ScanReport*)h->pin_scan)->bad[k];
+  const unsigned long long none = ~0ull;
   if (bad[0] != none || bad[1] != none || bad[2] != none) {
     // name the instance and bead / molecule of the first offender
     for (int g = 0; g < h->n_inst; ++g) {
@@ -2080,25 +2143,16 @@ int remc_upload_state(remc_handle* h, const float* pos, const float* rel, const 
     }
     return set_error(REMC_ERR_INVALID, "invalid state");
   }
-  state_pack_kernel<<<grid, 256, 0, h->stream>>>(sp, sr, sc, h->d_bead_info, (long long)nb,
-                                                 (long long)nm, h->d_pos, h->d_rel, h->d_centre);
+  state_pack_kernel<<<h->num_sms * 4, 256, 0, h->stream>>>(
+      sp, sr, sc, reinterpret_cast<const double2*>(h->d_stage_q), h->d_bead_info, fold, (long long)nb,
+      (long long)nm, h->n_sys, h->d_pos, h->d_rel, h->d_centre, reinterpret_cast<double2*>(h->d_quat),
+      h->d_sys);
   REMC_CUDA_TRY(cudaGetLastError());
-  fold_part_kernel<<<h->n_inst, 256, 0, h->stream>>>(h->d_sys, h->d_inst_sys, h->d_pos,
-                                                     h->d_rel, h->d_fold_part);
-  REMC_CUDA_TRY(cudaGetLastError());
-  fold_flag_kernel<<<h->n_sys, 256, 0, h->stream>>>(h->d_sys, h->d_fold_part);
-  REMC_CUDA_TRY(cudaGetLastError());
-  REMC_CUDA_TRY(cudaMemcpyAsync(h->d_quat, h->d_stage_q, sizeof(double) * 4 * nm,
-                                cudaMemcpyDeviceToDevice, h->stream));
   // the sweep folds the minimum image where every system allows it
-  std::vector<SysDev> sd(h->n_sys);
-  REMC_CUDA_TRY(cudaMemcpyAsync(sd.data(), h->d_sys, sizeof(SysDev) * h->n_sys,
-                                cudaMemcpyDeviceToHost, h->stream));
-  REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  bool fold = true;
-  for (const SysDev& S : sd) fold = fold && S.fold_mi;
-  if (fold != h->all_fold) h->config_gen++;  // a captured graph holds the other kernel
-  h->all_fold = fold;
+  bool all_fold = true;
+  for (int q = 0; q < h->n_sys; ++q) all_fold = all_fold && ((volatile ScanReport*)h->pin_scan)->fold[q];
+  if (all_fold != h->all_fold) h->config_gen++;  // a captured graph holds the other kernel
+  h->all_fold = all_fold;
   h->state_set = true;
   return REMC_OK;
 }
@@ -2168,20 +2222,18 @@ int remc_energy_full(remc_handle* h, double* out) {
   if (!h) return set_error(REMC_ERR_INVALID, "null handle");
   if (!h->tables_set || !h->state_set) return set_error(REMC_ERR_STATE, "tables/state not set");
   int grid = std::min(h->n_items, h->num_sms * 8);
-  REMC_CUDA_TRY(cudaMemsetAsync(h->d_energy_queue, 0, sizeof(int), h->stream));
   energy_tile_kernel<<<grid, kTile, 0, h->stream>>>(
       h->d_sys, h->d_inst_sys, h->d_pos, h->d_tab, h->d_mol_start, h->d_items_by_cost,
-      h->n_items, h->d_energy_queue, h->d_scratch, h->d_scratch_cc, consts_of(h), h->d_err);
+      h->n_items, h->d_energy_queue, h->d_scratch, h->d_scratch_cc, consts_of(h), h->pin_err);
   REMC_CUDA_TRY(cudaGetLastError());
   energy_reduce_kernel<<<(h->n_inst + 7) / 8, 256, 0, h->stream>>>(
-      h->d_item_off, h->n_inst, h->d_scratch, h->d_scratch_cc, h->d_energy, h->d_ecc);
+      h->d_item_off, h->n_inst, h->d_scratch, h->d_scratch_cc, h->d_energy, h->d_ecc,
+      out ? h->pin_energy : nullptr, h->d_energy_queue);
   REMC_CUDA_TRY(cudaGetLastError());
-  if (out) {
-    REMC_CUDA_TRY(cudaMemcpyAsync(out, h->d_energy, sizeof(double) * h->n_inst,
-                                  cudaMemcpyDeviceToHost, h->stream));
-    return check_device_error(h);
-  }
-  return REMC_OK;
+  if (!out) return REMC_OK;
+  const int rc = check_device_error(h);
+  memcpy(out, h->pin_energy, sizeof(double) * h->n_inst);
+  return rc;
 }
 
 int remc_get_energies(remc_handle* h, double* out) {
@@ -2214,6 +2266,7 @@ int remc_sweep_plain(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0)
   if (rc) return rc;
   if (n_steps < 0) return set_error(REMC_ERR_INVALID, "n_steps < 0");
   if (h->sweep_shape.csize > 1) {  // single CTAs all the same
+    if (allow_smem(h, false, !h->beads_in_smem)) return REMC_ERR_CUDA;
     rc = ensure_sweep_scratch(h, base_shape(h, h->sweep_threads, h->mol_in_smem, 1, h->beads_in_smem));
     if (rc) return rc;
   }
@@ -2772,7 +2825,7 @@ int remc_check_wait_timeout(remc_handle* h, int polls) {
   if (!h) return set_error(REMC_ERR_INVALID, "null handle");
   if (polls < 1 || polls > (1 << 20))
     return set_error(REMC_ERR_INVALID, "polls must be in [1, 2^20]");
-  wait_probe_kernel<<<1, 32, 0, h->stream>>>(h->d_err, polls);
+  wait_probe_kernel<<<1, 32, 0, h->stream>>>(h->pin_err, polls);
   REMC_CUDA_TRY(cudaGetLastError());
   return check_device_error(h);
 }
