@@ -1039,38 +1039,154 @@ __global__ void __launch_bounds__(kTile, 8) adjoint_tile_kernel(
   }
 }
 
-// Per-molecule force and torque about the centre (torque = sum rel x F):
-// one thread per molecule, grid (instance, molecule chunk). A one-bead
-// molecule is a copy widened to FP64; a chain's thread sums its beads in
-// order (FP64). Memory-bound: forces, rel and the six doubles per molecule.
+// Per-molecule force and torque about the centre (torque = sum rel x F), grid
+// (instance, molecule chunk): a lane per molecule; a one-bead molecule is a
+// copy widened to FP64, and the warp takes its longer molecules one at a time,
+// lanes over the beads (a thread per chain had left one thread walking 76
+// beads at memory latency while the rest waited: 23 us for 32 replicas, most
+// of the call's device time beside the pair kernel).
 __global__ void __launch_bounds__(128) molecule_force_torque_kernel(
     const SysDev* __restrict__ sys, const int* __restrict__ inst_sys,
     const int* __restrict__ mol_start, const float4* __restrict__ rel,
     const float* __restrict__ forces, double* __restrict__ out) {
-  const int inst = blockIdx.x;
+  const int inst = blockIdx.x, lane = threadIdx.x & 31;
   const SysDev S = sys[inst_sys[inst]];
   const int m = blockIdx.y * blockDim.x + threadIdx.x;
-  if (m >= S.n_mol) return;
   const int slot = inst - S.inst0;
-  const int base = S.bead_base + slot * S.n_beads;
-  const int* ms = mol_start + S.mstart_off;
-  const int a = ms[m], b = ms[m + 1];
-  double fx = 0.0, fy = 0.0, fz = 0.0, tx = 0.0, ty = 0.0, tz = 0.0;
-  for (int k = a; k < b; ++k) {
-    const float4 rl = rel[base + k];
-    const double Fx = forces[3 * (size_t)(base + k)], Fy = forces[3 * (size_t)(base + k) + 1],
-                 Fz = forces[3 * (size_t)(base + k) + 2];
-    fx += Fx;
-    fy += Fy;
-    fz += Fz;
-    tx += (double)rl.y * Fz - (double)rl.z * Fy;
-    ty += (double)rl.z * Fx - (double)rl.x * Fz;
-    tz += (double)rl.x * Fy - (double)rl.y * Fx;
+  const size_t base = S.bead_base + (size_t)slot * S.n_beads;
+  double* const o0 = out + 6 * (S.mol_base + (size_t)slot * S.n_mol);
+  int a = 0, n = 0;
+  if (m < S.n_mol) {
+    a = mol_start[S.mstart_off + m];
+    n = mol_start[S.mstart_off + m + 1] - a;
   }
-  double2* o = reinterpret_cast<double2*>(out + 6 * (size_t)(S.mol_base + slot * S.n_mol + m));
-  o[0] = make_double2(fx, fy);
-  o[1] = make_double2(fz, tx);
-  o[2] = make_double2(ty, tz);
+  struct Sum {
+    double v[6];
+  };
+  auto bead = [&](size_t k, Sum& t) {
+    const float4 rl = rel[k];
+    const double Fx = forces[3 * k], Fy = forces[3 * k + 1], Fz = forces[3 * k + 2];
+    t.v[0] += Fx;
+    t.v[1] += Fy;
+    t.v[2] += Fz;
+    t.v[3] += (double)rl.y * Fz - (double)rl.z * Fy;
+    t.v[4] += (double)rl.z * Fx - (double)rl.x * Fz;
+    t.v[5] += (double)rl.x * Fy - (double)rl.y * Fx;
+  };
+  auto put = [&](int q, const Sum& t) {
+    double2* o = reinterpret_cast<double2*>(o0 + 6 * (size_t)q);
+    o[0] = make_double2(t.v[0], t.v[1]);
+    o[1] = make_double2(t.v[2], t.v[3]);
+    o[2] = make_double2(t.v[4], t.v[5]);
+  };
+  if (n == 1) {
+    Sum t = {};
+    bead(base + a, t);
+    put(m, t);
+  }
+  for (unsigned longer = __ballot_sync(0xffffffffu, n > 1); longer; longer &= longer - 1) {
+    const int q = __ffs(longer) - 1;
+    const int a0 = __shfl_sync(0xffffffffu, a, q), n0 = __shfl_sync(0xffffffffu, n, q);
+    Sum t = {};
+    for (int k = lane; k < n0; k += 32) bead(base + a0 + k, t);
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      for (int off = 16; off > 0; off >>= 1) t.v[c] += __shfl_xor_sync(0xffffffffu, t.v[c], off);
+    if (lane == q) put(m, t);
+  }
+}
+
+// Raw contact table and offset, for derivatives by lambda: eps = lambda (M - e0).
+struct ContactTable {
+  float m[kNumAmino * kNumAmino];
+  float e0;
+};
+
+// From the per-type-pair sums G_ab of an instance: dE/dlambda = sum G_ab (M_ab -
+// e0), and, in place of G, dE/deps. The parameter is symmetric, eps_ab = eps_ba:
+// both entries carry the full derivative. One CTA per instance.
+__global__ void __launch_bounds__(128) deps_kernel(double* __restrict__ G, double* __restrict__ dl,
+                                                   const __grid_constant__ ContactTable T) {
+  constexpr int n = kNumAmino * kNumAmino;
+  __shared__ double s_g[n], s_red[4];
+  double* g = G + (size_t)blockIdx.x * n;
+  const int tid = threadIdx.x;
+  double v = 0.0;
+  for (int k = tid; k < n; k += 128) {
+    s_g[k] = g[k];
+    v += s_g[k] * ((double)T.m[k] - (double)T.e0);
+  }
+  v = warp_sum(v);
+  if ((tid & 31) == 0) s_red[tid >> 5] = v;
+  __syncthreads();
+  if (tid == 0) dl[blockIdx.x] = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
+  for (int k = tid; k < n; k += 128) {
+    const int a = k / kNumAmino, b = k % kNumAmino;
+    g[k] = a == b ? s_g[k] : s_g[k] + s_g[b * kNumAmino + a];
+  }
+}
+
+// dE/dlambda alone (the sensitivities' call): only residue pairs depend on
+// lambda, so the tiles are those of the chains. The per-type-pair sums are the
+// adjoint kernel's, term for term and tile for tile (lane L takes eight beads j
+// in the order q ^ r there, which is kept), and go into dE/dlambda at the end of
+// the tile. Grid (tile pair, instance); a crowded system of 500 beads has one
+// tile pair instead of ten: 31 us a call for 32 replicas, from 99 with the whole
+// adjoint, a copy of the sums and a loop on the host.
+__global__ void __launch_bounds__(kTile) lambda_tile_kernel(
+    const SysDev* __restrict__ sys, const int* __restrict__ inst_sys,
+    const float4* __restrict__ pos, const float4* __restrict__ tab,
+    const int* __restrict__ mol_start, float c_lj, double* __restrict__ dl, int inst0,
+    const __grid_constant__ ContactTable T) {
+  const int inst = inst0 + blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const SysDev S = sys[inst_sys[inst]];
+  const int ncb = S.n_chain_beads, nt = (ncb + kTile - 1) / kTile;
+  int ti = 0, tj = blockIdx.x;  // row ti holds nt - ti tiles
+  while (ti < nt && tj >= nt - ti) tj -= nt - ti++;
+  if (ti >= nt) return;
+  tj += ti;
+  __shared__ float4 s_j[kTile];
+  __shared__ float2 s_tab[kNumAmino * kNumAmino];  // sigma^2, repulsive-branch threshold
+  __shared__ float s_G[kNumAmino * kNumAmino];
+  const size_t base = S.bead_base + (size_t)(inst - S.inst0) * S.n_beads;
+  const int j0 = tj * kTile, jn = min(kTile, ncb - j0);
+  if (tid < jn) s_j[tid] = pos[base + j0 + tid];
+  for (int k = tid; k < kNumAmino * kNumAmino; k += kTile) {
+    const float4 t = tab[(k / kNumAmino) * kNT + k % kNumAmino];
+    s_tab[k] = make_float2(t.y, t.z);
+    s_G[k] = 0.0f;
+  }
+  __syncthreads();
+  const int i = ti * kTile + tid;
+  {
+    const float4 pi = i < ncb ? pos[base + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int ta = bead_type(pi.w);
+    // later beads of other molecules: from the own molecule's end on
+    const int lo = i < ncb ? max(mol_start[S.mstart_off + bead_mol(pi.w) + 1], i + 1) - j0 : jn;
+    const int r = (lane >> 2) & 7;
+    for (int jg = ti == tj ? (tid & ~31) : 0; jg < jn; jg += 8)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int j = jg + (q ^ r);
+        if (j < lo || j >= jn) continue;
+        const float4 pj = s_j[j];
+        const int e = ta * kNumAmino + bead_type(pj.w);
+        const float2 t = s_tab[e];
+        const float r2 = pair_r2(pi, pj, S.box, S.invbox);
+        const float rinv = fast_rsqrt(r2);
+        const float s2 = t.x * (rinv * rinv);
+        const float s6 = s2 * s2 * s2;
+        float dg = 4.0f * fmaf(-s6, s6, s6);
+        dg = r2 < t.y ? 2.0f - dg : dg;
+        atomicAdd(&s_G[e], dg * c_lj);
+      }
+  }
+  __syncthreads();
+  double acc = 0.0;
+  for (int k = tid; k < kNumAmino * kNumAmino; k += kTile)
+    acc += (double)s_G[k] * ((double)T.m[k] - (double)T.e0);
+  acc = warp_sum(acc);
+  if (lane == 0 && acc != 0.0) atomicAdd(&dl[inst], acc);
 }
 
 // ------------------------------------------------------------------ exchange
@@ -1256,6 +1372,7 @@ struct remc_handle {
   double* d_dxi = nullptr;
   double* d_eadj = nullptr;
   double* d_mft = nullptr;
+  double* d_dl = nullptr;  // dE/dlambda
   double* d_ecc = nullptr;
   int* d_n_samples = nullptr;
   int* d_n_bound = nullptr;
@@ -1311,7 +1428,7 @@ void free_all(remc_handle* h) {
                   h->d_evals_kh, h->d_evals_crowd, h->d_mol_role, h->d_mrole_off, h->d_recs,
                   h->d_queue,      h->d_scratch_cc, h->d_ecc,     h->d_n_samples,  h->d_n_bound,
                   h->d_sample_out, h->d_pose_out, h->d_sample_cursor, h->d_adj_acc,
-                  h->d_mft,
+                  h->d_mft,      h->d_dl,
                   h->d_ctrl,     h->d_items_by_cost, h->d_energy_queue,
                   h->d_item_off,   h->d_scratch,    h->d_newpos,
                   h->d_dE,       h->d_bead_info, h->d_stage,      h->d_stage_q,
@@ -2469,7 +2586,30 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   NvtxRange nvtx_range("remc_energy_adjoint");
   if (!h) return set_error(REMC_ERR_INVALID, "null handle");
   if (!h->tables_set || !h->state_set) return set_error(REMC_ERR_STATE, "tables/state not set");
+  ContactTable table;
+  memcpy(table.m, h->pair_table, sizeof(table.m));
+  table.e0 = h->params.e0;
+  const float c_lj = (float)((double)h->params.lj_cf * (double)h->params.kbt_cf);
   int rc = REMC_OK;
+  if (!h->d_dl && (rc = dev_alloc(&h->d_dl, h->n_inst))) return rc;
+  if (dE_dlambda && !forces && !mol_force_torque && !dE_dxi && !dE_deps && !energy) {
+    int nt = 0;
+    for (const SysDev& S : h->h_sys) nt = std::max(nt, (S.n_chain_beads + kTile - 1) / kTile);
+    REMC_CUDA_TRY(cudaMemsetAsync(h->d_dl, 0, sizeof(double) * h->n_inst, h->stream));
+    if (nt > 0) {
+      for (int g = 0; g < h->n_inst; g += 32768) {  // grid rows are limited
+        const int n = std::min(32768, h->n_inst - g);
+        lambda_tile_kernel<<<dim3(nt * (nt + 1) / 2, n), kTile, 0, h->stream>>>(
+            h->d_sys, h->d_inst_sys, h->d_pos, h->d_tab, h->d_mol_start, c_lj, h->d_dl, g, table);
+        REMC_CUDA_TRY(cudaGetLastError());
+      }
+    }
+    REMC_CUDA_TRY(cudaMemcpyAsync(h->pin_energy, h->d_dl, sizeof(double) * h->n_inst,
+                                  cudaMemcpyDeviceToHost, h->stream));
+    REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    memcpy(dE_dlambda, h->pin_energy, sizeof(double) * h->n_inst);
+    return REMC_OK;
+  }
   if (!h->d_adj_acc) {
     // forces first, every part on a 256-byte boundary
     auto up256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -2493,7 +2633,7 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   AdjConsts C;
   C.inv_xi = 1.0f / h->params.debye_length;
   C.inv_xi2 = C.inv_xi * C.inv_xi;
-  C.c_lj = (float)((double)h->params.lj_cf * (double)h->params.kbt_cf);
+  C.c_lj = c_lj;
   const bool cut = h->params.crowder_cutoff > 0.0f;
   auto adj = h->params.crowder_mode ? (cut ? adjoint_tile_kernel<true, true>
                                            : adjoint_tile_kernel<true, false>)
@@ -2512,6 +2652,10 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   molecule_force_torque_kernel<<<dim3(h->n_inst, (h->mmax + 127) / 128), 128, 0, h->stream>>>(
       h->d_sys, h->d_inst_sys, h->d_mol_start, h->d_rel, h->d_forces, h->d_mft);
   REMC_CUDA_TRY(cudaGetLastError());
+  if (dE_deps || dE_dlambda) {
+    deps_kernel<<<h->n_inst, 128, 0, h->stream>>>(h->d_G, h->d_dl, table);
+    REMC_CUDA_TRY(cudaGetLastError());
+  }
   if (forces)
     REMC_CUDA_TRY(cudaMemcpyAsync(forces, h->d_forces, sizeof(float) * 3 * h->total_beads,
                                   cudaMemcpyDeviceToHost, h->stream));
@@ -2524,29 +2668,14 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   if (energy)
     REMC_CUDA_TRY(cudaMemcpyAsync(energy, h->d_eadj, sizeof(double) * h->n_inst,
                                   cudaMemcpyDeviceToHost, h->stream));
-  std::vector<double> G;
-  if (dE_deps || dE_dlambda) {
-    G.resize((size_t)kNumAmino * kNumAmino * h->n_inst);
-    REMC_CUDA_TRY(cudaMemcpyAsync(G.data(), h->d_G, sizeof(double) * G.size(),
+  if (dE_dlambda)
+    REMC_CUDA_TRY(cudaMemcpyAsync(dE_dlambda, h->d_dl, sizeof(double) * h->n_inst,
                                   cudaMemcpyDeviceToHost, h->stream));
-  }
+  if (dE_deps)
+    REMC_CUDA_TRY(cudaMemcpyAsync(dE_deps, h->d_G,
+                                  sizeof(double) * kNumAmino * kNumAmino * (size_t)h->n_inst,
+                                  cudaMemcpyDeviceToHost, h->stream));
   REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  // symmetric parameter eps_ab = eps_ba: both table entries carry the full
-  // derivative; eps = lambda (M - e0) gives dE/dlambda = sum G_ab (M_ab - e0)
-  for (int g = 0; g < h->n_inst && !G.empty(); ++g) {
-    const double* Gi = &G[(size_t)g * kNumAmino * kNumAmino];
-    double dl = 0.0;
-    for (int a = 0; a < kNumAmino; ++a) {
-      for (int b = 0; b < kNumAmino; ++b) {
-        const double d = (a == b) ? Gi[a * kNumAmino + a]
-                                  : Gi[a * kNumAmino + b] + Gi[b * kNumAmino + a];
-        if (dE_deps) dE_deps[(size_t)g * kNumAmino * kNumAmino + a * kNumAmino + b] = d;
-        dl += Gi[a * kNumAmino + b] *
-              ((double)h->pair_table[a * 20 + b] - (double)h->params.e0);
-      }
-    }
-    if (dE_dlambda) dE_dlambda[g] = dl;
-  }
   return REMC_OK;
 }
 
