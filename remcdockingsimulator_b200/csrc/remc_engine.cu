@@ -28,6 +28,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -136,14 +137,21 @@ __global__ void __launch_bounds__(256) proposal_kernel(ProposalArgs P) {
 // instance, the pair evaluations of its n_steps records plus `step_cost` per
 // step for the step's fixed work (record, reduction, barrier, decision); a
 // one-bead rotation has no pairs. Integer sums, so the result does not depend
-// on the order of the additions. One CTA per instance.
+// on the order of the additions. One CTA per instance. Instances that run on
+// clusters of their own come first, before the queue's.
 __global__ void __launch_bounds__(256) block_cost_kernel(const SysDev* __restrict__ sys,
                                                          const int* __restrict__ inst_sys,
                                                          const StepRec* __restrict__ recs,
                                                          int rec_stride, int n_steps,
                                                          long long step_cost,
+                                                         const float* __restrict__ sys_cost,
+                                                         float apart_from,
                                                          long long* __restrict__ cost) {
   const int inst = blockIdx.x;
+  if (sys_cost[inst_sys[inst]] >= apart_from) {  // on clusters, not in the queue
+    if (threadIdx.x == 0) cost[inst] = LLONG_MAX;
+    return;
+  }
   const int N = sys[inst_sys[inst]].n_beads;
   const StepRec* r = recs + (size_t)inst * rec_stride;
   long long c = 0;
@@ -1393,6 +1401,14 @@ struct remc_handle {
   int sweep_threads = 128;  // virtual threads per CTA (the schedule's threads per replica)
   int sweep_block = 256;    // threads per CTA
   SweepShape sweep_shape{};
+  // costly systems apart: the first n_apart of inst_list run on clusters of
+  // their own beside the work queue
+  SweepShape apart_shape{};
+  int n_apart = 0;
+  float apart_from = INFINITY;       // expected cost of their systems, at least
+  std::vector<float> sys_cost;       // expected cycles per step, by system
+  std::vector<float> sys_chain_cost; // of them, in chain steps' pairs
+  float* d_sys_cost = nullptr;
   bool all_fold = false;    // every system's fold flag is set (the state uploaded last)
   int nrel = 0;             // beads up to the last one of a molecule of several
   bool any_crowders = false;
@@ -1432,7 +1448,7 @@ void free_all(remc_handle* h) {
                   h->d_ctrl,     h->d_items_by_cost, h->d_energy_queue,
                   h->d_item_off,   h->d_scratch,    h->d_newpos,
                   h->d_dE,       h->d_bead_info, h->d_stage,      h->d_stage_q,
-                  h->d_sweep_scratch, h->d_scan_part, h->d_scan};
+                  h->d_sweep_scratch, h->d_scan_part, h->d_scan, h->d_sys_cost};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->h_pin) cudaFreeHost(h->h_pin);
@@ -1642,6 +1658,50 @@ int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* cl
   return REMC_OK;
 }
 
+// Cycles of sweep work on half an SM (two CTAs of 256 threads on each), from
+// per-replica clocks on the 64-system batch: a residue pair's and a wall pair's
+// change, the rest of a chain step, a one-bead step in a group of some seven.
+constexpr double kResiduePairCycles = 1.2, kWallPairCycles = 0.65, kChainStepCycles = 6000.0;
+constexpr double kOneBeadCycles = 900.0, kOneBeadPairCycles = 1.1;
+
+// Which systems run apart, each replica on a cluster of four CTAs, because the
+// block would otherwise end in their replicas alone: in a batch of unlike
+// systems one with few crowders moves a chain in every third step and takes
+// longer than the whole batch does on average. The prefix of the systems by
+// cost that makes the expected end earliest: the later of the SM slots' mean
+// load and the longest replica, where a cluster takes the chain steps' pairs in
+// a third of the time, all else in 1.2 times it, and four slots. A batch of 64
+// systems ran 15.1 ms per 1000 steps without it (its balanced load is 10.9),
+// 12.3 with four systems apart; every replica on a cluster took 21.9 where
+// none took 15.9.
+void choose_apart(remc_handle* h, int slots) {
+  std::vector<int> order(h->n_sys);
+  for (int q = 0; q < h->n_sys; ++q) order[q] = q;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->sys_cost[a] > h->sys_cost[b]; });
+  double load = 0.0;
+  for (int q = 0; q < h->n_sys; ++q) load += (double)h->sys_cost[q] * h->h_sys[q].n_rep;
+  double best = 0.9 * std::max(load / slots, (double)h->sys_cost[order[0]]), longest = 0.0;
+  int n = 0;
+  h->n_apart = 0;
+  h->apart_from = INFINITY;
+  for (int k = 0; k < h->n_sys; ++k) {
+    const int q = order[k];
+    const double t = h->sys_cost[q], c = h->sys_chain_cost[q];
+    const double apart = c / 3.3 + 1.2 * (t - c);
+    longest = std::max(longest, apart);
+    load += (4.0 * apart - t) * h->h_sys[q].n_rep;
+    n += h->h_sys[q].n_rep;
+    if (k + 1 < h->n_sys && h->sys_cost[order[k + 1]] == h->sys_cost[q]) continue;
+    const double rest = k + 1 < h->n_sys ? h->sys_cost[order[k + 1]] : 0.0;
+    const double end = std::max(load / slots, std::max(longest, rest));
+    if (end < best) {
+      best = end;
+      h->n_apart = n;
+      h->apart_from = h->sys_cost[q];
+    }
+  }
+}
+
 // Set the sweep schedule: virtual threads per CTA (they fix the order of the
 // sums, see remc_sweep.cuh), where molecule data lives, CTAs per replica, and
 // whether the beads are resident in shared memory.
@@ -1682,6 +1742,20 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
     }
   }
   h->sweep_cluster_slots = clusters;
+  h->n_apart = 0;
+  h->apart_from = INFINITY;
+  SweepShape apart = base_shape(h, threads, mol_in_smem, 4, beads_in_smem);
+  apart.vsize = 1;
+  apart.aj_in_smem = 1;
+  if (shape.csize == 1 && beads_in_smem && SweepSmem::make(apart).total <= (size_t)h->max_dyn_smem) {
+    choose_apart(h, per_sm * h->num_sms);
+    int n = 0, k = 0;
+    if (h->n_apart && (fit_sweep(h, apart, block, &n, &k) || ensure_sweep_scratch(h, apart))) {
+      h->n_apart = 0;
+      h->apart_from = INFINITY;
+    }
+    h->apart_shape = apart;
+  }
   if (ensure_sweep_scratch(h, shape)) return REMC_ERR_NOMEM;
   h->sweep_shape = shape;
   h->sweep_threads = threads;
@@ -1728,22 +1802,23 @@ int launch_proposals(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0,
   return REMC_OK;
 }
 
+// How a sweep kernel runs: single CTAs on the replicas of the list, each once;
+// single CTAs on a work queue; a cluster per replica; or the queue beside the
+// clusters launched just before (it may start once all of them have, and ends
+// after them).
+enum class SweepRun { kOnce, kQueue, kClusters, kQueueBeside };
+
 int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* inst_list,
-                        int n_blocks, bool persistent, uint32_t step0, const uint32_t* ctrl) {
+                        int n_blocks, SweepRun run, const SweepShape& shape, uint32_t step0,
+                        const uint32_t* ctrl) {
   SweepArgs A;
   A.sys = h->d_sys;
   A.inst_sys = h->d_inst_sys;
   A.inst_list = inst_list;
-  // a cluster schedule runs one cluster per replica (no work queue); the
-  // one-replica-per-launch path always runs single CTAs
-  const int csize = persistent ? h->sweep_shape.csize : 1;
-  if (csize > 1) persistent = false;
-  A.queue = persistent ? h->d_queue : nullptr;
+  const bool queue = run == SweepRun::kQueue || run == SweepRun::kQueueBeside;
+  A.queue = queue ? h->d_queue : nullptr;
   A.n_list = n_blocks;
-  if (persistent) {
-    REMC_CUDA_TRY(cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream));
-    n_blocks = std::min(n_blocks, h->sweep_grid);
-  }
+  if (queue) n_blocks = std::min(n_blocks, h->sweep_grid);
   A.pos = h->d_pos;
   A.rel = h->d_rel;
   A.centre = h->d_centre;
@@ -1774,32 +1849,30 @@ int launch_sweep_kernel(remc_handle* h, int n_steps, int rec_offset, const int* 
   A.rec_stride = (int)h->recs_cap;
   A.rec_offset = rec_offset;
   A.n_steps = n_steps;
-  A.shape = csize == h->sweep_shape.csize
-                ? h->sweep_shape
-                : base_shape(h, h->sweep_threads, h->mol_in_smem, csize, h->beads_in_smem);
+  A.shape = shape;
   A.scratch = h->d_sweep_scratch;
-  A.scratch_stride = (long long)scratch_stride(A.shape);
+  A.scratch_stride = (long long)scratch_stride(shape);
   A.K = consts_of(h);
-  const bool gb = !h->beads_in_smem;
-  const size_t smem = SweepSmem::make(A.shape).total;
-  if (csize == 1) {
-    sweep_fn(h, false, gb)<<<n_blocks, h->sweep_block, smem, h->stream>>>(A);
-  } else {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+  const int csize = shape.csize;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(csize * n_blocks);
+  cfg.blockDim = dim3(h->sweep_block);
+  cfg.dynamicSmemBytes = SweepSmem::make(shape).total;
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  if (csize > 1) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = csize;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(csize * n_blocks);
-    cfg.blockDim = dim3(h->sweep_block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = h->stream;
-    cfg.attrs = attr;
     cfg.numAttrs = 1;
-    REMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, sweep_fn(h, true, gb), A));
+  } else if (run == SweepRun::kQueueBeside) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 1;
   }
-  REMC_CUDA_TRY(cudaGetLastError());
+  REMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, sweep_fn(h, csize > 1, !shape.beads_in_smem), A));
   return REMC_OK;
 }
 
@@ -1811,7 +1884,7 @@ constexpr long long kStepCostPerThread = 6;
 
 // The persistent sweep takes its work in cost order (remc_set_work_order).
 bool uses_cost_order(const remc_handle* h) {
-  return h->work_order == 1 && h->sweep_csize == 1 && h->n_inst > 1 &&
+  return h->work_order == 1 && h->sweep_shape.csize == 1 && h->n_inst > 1 &&
          h->n_inst <= kMaxRankedInst;
 }
 
@@ -1821,20 +1894,30 @@ int launch_sweep(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0,
                  const uint32_t* ctrl) {
   int rc = launch_proposals(h, n_steps, seed, step0, ctrl);
   if (rc) return rc;
+  if (h->sweep_shape.csize > 1)  // one cluster per replica
+    return launch_sweep_kernel(h, n_steps, 0, h->d_inst_list, h->n_inst, SweepRun::kClusters,
+                               h->sweep_shape, step0, ctrl);
   // the work queue in decreasing order of what each replica's proposals cost
-  // (single CTAs per replica: a cluster schedule runs every replica at once)
   const int* list = h->d_inst_list;
   if (uses_cost_order(h) && n_steps > 0) {
     block_cost_kernel<<<h->n_inst, 256, 0, h->stream>>>(
         h->d_sys, h->d_inst_sys, h->d_recs, (int)h->recs_cap, n_steps,
-        kStepCostPerThread * (long long)h->sweep_threads, h->d_inst_cost);
+        kStepCostPerThread * (long long)h->sweep_threads, h->d_sys_cost, h->apart_from, h->d_inst_cost);
     REMC_CUDA_TRY(cudaGetLastError());
     rank_kernel<<<(h->n_inst + 7) / 8, 256, 0, h->stream>>>(h->d_inst_cost, h->n_inst,
                                                              h->d_inst_order);
     REMC_CUDA_TRY(cudaGetLastError());
     list = h->d_inst_order;
   }
-  return launch_sweep_kernel(h, n_steps, 0, list, h->n_inst, true, step0, ctrl);
+  REMC_CUDA_TRY(cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->stream));
+  if (!h->n_apart)
+    return launch_sweep_kernel(h, n_steps, 0, list, h->n_inst, SweepRun::kQueue, h->sweep_shape, step0,
+                               ctrl);
+  rc = launch_sweep_kernel(h, n_steps, 0, h->d_inst_list, h->n_apart, SweepRun::kClusters,
+                           h->apart_shape, step0, ctrl);
+  if (rc || h->n_apart == h->n_inst) return rc;
+  return launch_sweep_kernel(h, n_steps, 0, list + h->n_apart, h->n_inst - h->n_apart,
+                             SweepRun::kQueueBeside, h->sweep_shape, step0, ctrl);
 }
 
 }  // namespace
@@ -1992,6 +2075,24 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   }
   const int max_dyn = max_smem - (int)fattr.sharedSizeBytes;
   h->max_dyn_smem = max_dyn;
+  for (const SysDev& S : h->h_sys) {
+    const int* ms = &h->h_mol_start[S.mstart_off];
+    const double ncb = S.n_chain_beads, N = S.n_beads;
+    double chain = 0.0, other = 0.0;
+    for (int m = 0; m < S.n_mol; ++m) {
+      const double n = ms[m + 1] - ms[m];
+      const bool crowd = ms[m] >= S.n_chain_beads;
+      if (n > 1 || !crowd) {
+        chain += n * (crowd ? kWallPairCycles * (N - n)
+                            : kResiduePairCycles * (ncb - n) + kWallPairCycles * (N - ncb));
+        other += kChainStepCycles;
+      } else {
+        other += kOneBeadCycles + kOneBeadPairCycles * N;
+      }
+    }
+    h->sys_chain_cost.push_back((float)(chain / S.n_mol));
+    h->sys_cost.push_back((float)((chain + other) / S.n_mol));
+  }
   // default schedule (the autotuner may replace it): molecule data in shared
   // memory when it fits, more threads per replica for larger systems, and the
   // beads left in global memory for systems too large for shared memory
@@ -2044,25 +2145,15 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   std::vector<int> inst_list(h->n_inst);
   for (int g = 0; g < h->n_inst; ++g) inst_list[g] = g;
   // largest expected cost first (longest-processing-time order for the work
-  // queue): expected pair evaluations per step = sum_m n_m (N - n_m) / M
-  std::vector<double> sys_cost(h->n_sys, 0.0);
-  for (int s2 = 0; s2 < h->n_sys; ++s2) {
-    const SysDev& S = h->h_sys[s2];
-    const int* ms = &h->h_mol_start[S.mstart_off];
-    double c = 0.0;
-    for (int m = 0; m < S.n_mol; ++m) {
-      const double n = ms[m + 1] - ms[m];
-      c += n * (S.n_beads - n);
-    }
-    sys_cost[s2] = c / S.n_mol + S.n_beads;  // + per-step bookkeeping
-  }
+  // queue)
   std::stable_sort(inst_list.begin(), inst_list.end(), [&](int a, int b) {
-    return sys_cost[h->h_inst_sys[a]] > sys_cost[h->h_inst_sys[b]];
+    return h->sys_cost[h->h_inst_sys[a]] > h->sys_cost[h->h_inst_sys[b]];
   });
   if (!rc) rc = dev_alloc(&h->d_sys, h->h_sys.size());
   if (!rc) rc = dev_alloc(&h->d_inst_sys, h->n_inst);
   if (!rc) rc = dev_alloc(&h->d_inst_list, h->n_inst);
   if (!rc) rc = dev_alloc(&h->d_inst_cost, h->n_inst);
+  if (!rc) rc = dev_alloc(&h->d_sys_cost, h->n_sys);
   if (!rc) rc = dev_alloc(&h->d_inst_order, h->n_inst);
   if (!rc) rc = dev_alloc(&h->d_pos, h->total_beads);
   if (!rc) rc = dev_alloc(&h->d_bead_info, h->total_beads);
@@ -2126,6 +2217,7 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   up(h->d_sys, h->h_sys.data(), sizeof(SysDev) * h->h_sys.size());
   up(h->d_inst_sys, h->h_inst_sys.data(), sizeof(int) * h->n_inst);
   up(h->d_inst_list, inst_list.data(), sizeof(int) * h->n_inst);
+  up(h->d_sys_cost, h->sys_cost.data(), sizeof(float) * h->n_sys);
   up(h->d_mol_start, h->h_mol_start.data(), sizeof(int) * h->h_mol_start.size());
   up(h->d_mol_role, h->h_mol_role.data(), sizeof(int) * h->h_mol_role.size());
   std::vector<int> mrole_off(h->n_sys);
@@ -2382,9 +2474,11 @@ int remc_sweep_plain(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0)
   int rc = check_ready(h);
   if (rc) return rc;
   if (n_steps < 0) return set_error(REMC_ERR_INVALID, "n_steps < 0");
-  if (h->sweep_shape.csize > 1) {  // single CTAs all the same
+  SweepShape once = h->sweep_shape;
+  if (once.csize > 1) {  // single CTAs all the same
+    once = base_shape(h, h->sweep_threads, h->mol_in_smem, 1, h->beads_in_smem);
     if (allow_smem(h, false, !h->beads_in_smem)) return REMC_ERR_CUDA;
-    rc = ensure_sweep_scratch(h, base_shape(h, h->sweep_threads, h->mol_in_smem, 1, h->beads_in_smem));
+    rc = ensure_sweep_scratch(h, once);
     if (rc) return rc;
   }
   const size_t chunk_max = max_chunk_steps(h);
@@ -2398,7 +2492,7 @@ int remc_sweep_plain(remc_handle* h, int n_steps, uint64_t seed, uint32_t step0)
       for (int g = 0; g < h->n_inst; ++g) {
         // one single-CTA launch per replica per step; d_inst_list + g names one
         // instance (instances are independent within a step, so order is free)
-        rc = launch_sweep_kernel(h, 1, s, h->d_inst_list + g, 1, false,
+        rc = launch_sweep_kernel(h, 1, s, h->d_inst_list + g, 1, SweepRun::kOnce, once,
                                  step0 + (uint32_t)(done + s), nullptr);
         if (rc) return rc;
       }
@@ -2922,7 +3016,8 @@ int remc_set_work_order(remc_handle* h, int by_cost) {
 int remc_get_work_order(remc_handle* h, int* by_cost, int* launches_per_sweep) {
   if (!h) return set_error(REMC_ERR_INVALID, "null handle");
   if (by_cost) *by_cost = h->work_order;
-  if (launches_per_sweep) *launches_per_sweep = uses_cost_order(h) ? 4 : 2;
+  if (launches_per_sweep)
+    *launches_per_sweep = (uses_cost_order(h) ? 4 : 2) + (h->n_apart && h->n_apart < h->n_inst ? 1 : 0);
   return REMC_OK;
 }
 

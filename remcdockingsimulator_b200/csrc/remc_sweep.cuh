@@ -542,6 +542,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       __syncthreads();
   };
 
+  // a work queue launched beside these clusters may start once all have
+  if (CLUSTER) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
   for (int it = 0;; ++it) {
   int idx;
   if (A.queue) {
@@ -1229,8 +1232,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   }
   __syncthreads();  // shared memory is reused by the next instance
   }  // instance loop
-  // no CTA leaves while another may still write into its shared memory
-  if (CLUSTER) cooperative_groups::this_cluster().sync();
+  // no CTA leaves while another may still write into its shared memory; a work
+  // queue launched beside clusters ends after them
+  if (CLUSTER)
+    cooperative_groups::this_cluster().sync();
+  else
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 #endif  // __CUDACC__
