@@ -64,7 +64,8 @@ struct SamplePose {
 
 constexpr int kRing = 64;          // proposal records held in shared memory (two halves)
 constexpr int kLgGroup = 3;
-constexpr int kGroup = 1 << kLgGroup;  // most one-bead steps evaluated together
+constexpr int kGroup = 1 << kLgGroup;  // most one-bead moves evaluated together
+constexpr int kWindow = 2 * kGroup;    // most steps of a group, one-bead rotations among them
 constexpr int kSweepThreads = 512; // most threads of a sweep CTA
 constexpr int kSweepWarps = kSweepThreads / 32;
 
@@ -193,9 +194,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // ---- one-bead crowder steps, in groups
 //
 // A one-bead step is short (N pairs) against the fixed chain of a step: record,
-// reduction, barrier, decision. Up to kGroup consecutive one-bead crowder steps
-// are therefore evaluated at once, each by its own warps and against the state
-// before the group, and decided in order afterwards: step b's dE is its sum
+// reduction, barrier, decision. Up to kGroup one-bead crowder moves in a row
+// (rotations of one bead between them, which move nothing: dE = 0) are therefore
+// evaluated at once, each by its own warps and against the state before the
+// group, and decided in order afterwards: step b's dE is its sum
 // over that state, plus, for every earlier step a of the group that was
 // accepted, the change of its sum when bead a stands at its new place.
 //
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   double* const s_sums = reinterpret_cast<double*>(smem_raw + L.sums);
   float* const s_terms = reinterpret_cast<float*>(smem_raw + L.terms);
   __shared__ int s_next, s_done, s_bound, s_mask[2];
-  __shared__ double s_dE[2][kGroup];  // a group's dE by step, and which were accepted
+  __shared__ double s_dE[2][kWindow];  // a group's dE by step, and which were accepted
   __shared__ long long s_pose_slot;
 
   const int tid = threadIdx.x, nthr = blockDim.x;
@@ -637,11 +639,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (warp == 2 && (pending & 2)) {
       const int at = (pending & 1) ^ 1;
       const int accepted = s_mask[at];
-#pragma unroll 1
-      for (int k = 0; k < kGroup; ++k) {
-        const double d = s_dE[at][k];
-        if ((accepted >> k) & 1) energy += d;
-      }
+      for (int m = accepted; m; m &= m - 1) energy += s_dE[at][__ffs(m) - 1];
     }
     pending &= 1;
   };
@@ -718,31 +716,42 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     return make_float4(wrap_box(x0, box), wrap_box(x1, box), wrap_box(x2, box), c.w);
   };
   // What the next pass does, looked at ahead (it does not depend on the state):
-  // lane i's record of the steps from s on, and how many of them form a group
-  // (0: step s is not a one-bead crowder step). The group ends before another
-  // kind of step, at the sampling chunk's end and before a second bead of a
-  // virtual thread.
+  // lane i's record of the steps from s on, how many of them form a group (0:
+  // step s is not a one-bead crowder step), and which of them move their bead.
+  // The group ends before another kind of step, at the sampling chunk's end,
+  // before a second move in a virtual thread or a second rotation of a
+  // molecule, and before the move it has no warps for.
   int run = 0, my_m0 = 0, my_m = 0;
+  unsigned movers = 0u;
   bool my_rot = false;
   float my_t[3];
+  const int window = S.translate_only_crowders ? kGroup : kWindow;
   auto look = [&](int s, int readable, int chunk) {
-    const bool there = lane < kGroup && s + lane < readable && (chunk <= 0 || lane < chunk);
+    const bool there = lane < window && s + lane < readable && (chunk <= 0 || lane < chunk);
     const StepRec& r = s_ring[(there ? s + lane : s) & (kRing - 1)];
     my_m0 = r.m0;
     my_m = r.m;
-    my_rot = (r.info & kRecRotate) != 0;  // a one-bead crowder: moves nothing, dE = 0
+    my_rot = (r.info & kRecRotate) != 0;
     my_t[0] = r.t[0];
     my_t[1] = r.t[1];
     my_t[2] = r.t[2];
     const bool one = there && (r.info & kRecCrowd) && (r.info & kRecCount) == 1;
-    const int key = one ? (my_m0 & gmask) : -1 - lane;
-    bool stop = !one;  // lanes from kGroup on always stop it
-#pragma unroll
-    for (int k = 1; k < kGroup; ++k) {
+    const int key = !one ? -1 - lane : my_rot ? kRecRotate | my_m0 : my_m0 & gmask;
+    const unsigned moves = __ballot_sync(full, one && !my_rot);
+    const unsigned before = (1u << lane) - 1u;
+    // lanes from the window's end on always stop it
+    bool stop = !one || (!my_rot && __popc(moves & before) >= (1 << lg_most));
+    auto alike = [&](int k) {
       const int other = __shfl_up_sync(full, key, k);
       stop = stop || (lane >= k && other == key);
-    }
+    };
+#pragma unroll
+    for (int k = 1; k < kGroup; ++k) alike(k);
+    if (window > kGroup)
+#pragma unroll
+      for (int k = kGroup; k < kWindow; ++k) alike(k);
     run = __ffs(__ballot_sync(full, stop)) - 1;
+    movers = moves & ((1u << run) - 1u);
   };
 
   // Records up to `avail` can be read, up to `filled` are requested. The
@@ -762,9 +771,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       cp_async_commit();
       filled += nrec;
     }
-    // requested records are waited for well before they are read, and are
-    // visible after this pass's first barrier
-    const bool landing = filled != avail && s + 2 * kGroup >= avail;
+    // requested records are waited for, and visible, at this pass's barrier
+    const bool landing = filled != avail;
     if (alone) run = 0;
     alone = false;
     double* const sums = s_sums + parity * pass_sums(csize);
@@ -772,19 +780,27 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (CLUSTER) parity ^= 1;
 
     if (run > 0) {
-      // ---- a group of one-bead crowder steps: warp gw takes virtual warps
-      // [p VW, (p + 1) VW) of step s + b, gw = b P + p
-      const int gsize = min(run, 1 << lg_most);
+      // ---- a group of one-bead crowder steps. Lane i holds step s + i; move b
+      // of the group is that of lane at(b). Warp gw takes virtual warps [p VW,
+      // (p + 1) VW) of move b, gw = b P + p
+      const int gsize = run, n_moves = __popc(movers);
       const int b = gw >> lgP, p = gw & (P - 1);
+      int my_at = lane;  // lane b: the lane of move b
+      if (n_moves < gsize) {
+        unsigned m = movers;
+#pragma unroll
+        for (int k = 0; k < kGroup - 1; ++k)
+          if (k < lane) m &= m - 1u;
+        my_at = max(__ffs(m) - 1, 0);
+      }
       const float4 my_old = s_beads[my_m0];
       const float4 my_new = translated(at_centre ? my_old : cent[my_m], my_t);
-      const unsigned movers = __ballot_sync(full, !my_rot);
-      if (b < gsize) {
-        const int b_m0 = __shfl_sync(full, my_m0, b);
-        const bool b_rot = !((movers >> b) & 1u);
+      if (b < n_moves) {
+        const int at_b = __shfl_sync(full, my_at, b);
+        const int b_m0 = __shfl_sync(full, my_m0, at_b);
         const float4 po = s_beads[b_m0];
-        const float4 pn = make_float4(__shfl_sync(full, my_new.x, b), __shfl_sync(full, my_new.y, b),
-                                      __shfl_sync(full, my_new.z, b), 0.0f);
+        const float4 pn = make_float4(__shfl_sync(full, my_new.x, at_b), __shfl_sync(full, my_new.y, at_b),
+                                      __shfl_sync(full, my_new.z, at_b), 0.0f);
         GroupView G;
         G.beads = s_beads;
         G.row = s_tab + bead_type(po.w) * kNT;
@@ -797,16 +813,17 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
         G.cut2 = G.row[0].z;  // every entry of a crowder's row holds the cutoff
         G.box = box;
         G.invbox = invbox;
-        // corrections by earlier steps a = p, p + P, ...: a lane group each
+        // corrections by earlier moves a = p, p + P, ...: a lane group each
         const int a = ((lane >> lg_lanes) << lgP) + p;
-        const bool active = a < b && !b_rot && ((movers >> a) & 1u);
-        const int qa = __shfl_sync(full, my_m0, a & 31);
+        const bool active = a < b;
+        const int at_a = __shfl_sync(full, my_at, a & (kGroup - 1));
+        const int qa = __shfl_sync(full, my_m0, at_a);
         const float4 pa =
-            make_float4(__shfl_sync(full, my_new.x, a & 31), __shfl_sync(full, my_new.y, a & 31),
-                        __shfl_sync(full, my_new.z, a & 31), __shfl_sync(full, my_old.w, a & 31));
+            make_float4(__shfl_sync(full, my_new.x, at_a), __shfl_sync(full, my_new.y, at_a),
+                        __shfl_sync(full, my_new.z, at_a), __shfl_sync(full, my_old.w, at_a));
         double hi = 0.0, lo = 0.0, c_hi = 0.0, c_lo = 0.0;
         bool fits = true, c_fits = true;
-        if (!b_rot) {
+        {
           const MovedBead<R12, CUT, FOLD> mv(G, pn, po);
           auto split = [&](float x) {
             double h, l;
@@ -855,36 +872,39 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       // installs; meanwhile warp 2 adds up the last group's energies, the last
       // warp fetches rotations, and all but warp 0 look at the next steps
       const StepRec& mine = s_ring[(s + (lane < gsize ? lane : 0)) & (kRing - 1)];
+      const unsigned group_movers = movers;
       const bool turns = warp == nwarps - 1 && crank == 0 && lane < gsize && my_rot;
       double4 quat = make_double4(0.0, 0.0, 0.0, 0.0);
       double* const my_quat = A.quat + 4 * (size_t)(mol_off + my_m);
       if (turns) quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
       if (warp == 0) {
         double hi = 0.0, lo = 0.0;
-        if (lane < gsize)
+        const bool moves = lane < gsize && !my_rot;
+        const int my_b = __popc(group_movers & ((1u << lane) - 1u));  // moves before this lane's step
+        if (moves)
           for (int w = 0; w < P; ++w) {
-            const double2 x = *reinterpret_cast<const double2*>(sums + 2 * ((lane << lgP) + w));
+            const double2 x = *reinterpret_cast<const double2*>(sums + 2 * ((my_b << lgP) + w));
             hi += x.x;
             lo += x.y;
           }
-        // corrections by the earlier steps of the group that move their bead
+        // corrections by the earlier moves of the group
         const double2* const mine_c =
-            reinterpret_cast<const double2*>(sums + 2 * kSweepWarps * csize + lane * (lane - 1));
-        const unsigned use = (lane < gsize && !my_rot) ? movers & ((1u << lane) - 1u) : 0u;
+            reinterpret_cast<const double2*>(sums + 2 * kSweepWarps * csize + my_b * (my_b - 1));
         double2 c[kGroup - 1];
 #pragma unroll
-        for (int k = 0; k < kGroup - 1; ++k)
-          c[k] = ((use >> k) & 1u) ? mine_c[k] : make_double2(0.0, 0.0);
+        for (int k = 0; k < kGroup - 1; ++k) c[k] = moves && k < my_b ? mine_c[k] : make_double2(0.0, 0.0);
         const double thr = fmax(mine.thr, 0.0);  // accepted: dE < 0 or dE < thr
         double dE = hi + lo;
+        unsigned left_movers = group_movers;
 #pragma unroll
         for (int k = 0; k < kGroup - 1; ++k) {
           const unsigned accepted = __ballot_sync(full, dE < thr);
-          if ((accepted >> k) & 1u) {  // zero past the group's end
+          if (accepted & left_movers & (0u - left_movers)) {  // move k: the lowest left (none past the end)
             hi += c[k].x;
             lo += c[k].y;
             dE = hi + lo;
           }
+          left_movers &= left_movers - 1u;
         }
         // a sum that did not split (NaN) ends the group before its step, which
         // is then taken by itself
