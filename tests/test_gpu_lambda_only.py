@@ -25,7 +25,8 @@ def test_lambda_only_equals_adjoint(built_lib, chains, crowders):
         # 1e-5 of the sum of magnitudes; its own check against FP64 holds 1e-4
         scale = np.abs(full["dE_deps"]).sum(axis=(1, 2)) * 10.0 + 1e-12
         assert np.all(np.abs(only - full["dE_dlambda"]) <= 1e-5 * scale)
-        assert np.array_equal(only, eng.dE_dlambda()) or np.allclose(only, eng.dE_dlambda(), rtol=1e-12)
+        # the same FP32 sums over a tile again, by atomics in an order of their own
+        assert np.all(np.abs(only - eng.dE_dlambda()) <= 1e-5 * scale)
         g = full["dE_deps"]
         assert np.array_equal(g, np.swapaxes(g, 1, 2))
         raw = table.pairs.astype(np.float64).reshape(20, 20) - np.float64(np.float32(-2.27))
