@@ -964,6 +964,64 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (turns) quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
     const float4 c_old = cent[r.m];
     const float4 c_new = rot ? c_old : translated(c_old, r.t);
+    // bead at place x of the list of beads, the place y of its sum, and whether
+    // it counts. With one virtual CTA the list leaves the molecule out; else
+    // it holds this CTA's beads, the molecule's masked
+    auto bead_at = [&](int x, int& y, bool& counts) {
+      int j;
+      if (!CLUSTER || spread) {
+        j = x < m0 ? x : x + n;
+        y = j;
+        counts = true;
+      } else {
+        y = x;
+        j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
+        counts = (unsigned)(j - m0) >= (unsigned)n;
+      }
+      return j;
+    };
+    // places of the list below bead e
+    auto places = [&](int e) {
+      if (!CLUSTER || spread) return e <= m0 ? e : max(m0, e - n);
+      return ((e >> lgs) << lgv) + min(max((e & gmask) - vrank * vthr, 0), vthr);
+    };
+    // is crowder pair j the odd one of its virtual thread's last pass (see
+    // wall_term)? Alone in a pass: a one-residue chain's pairs, and the
+    // chain beads a moved crowder meets
+    auto odd_last = [&](int j) {
+      if (n == 1 || j < ncb) return true;
+      const int a = j < m0 ? ncb : max(m0 + n, ncb), e = j < m0 ? m0 : N;
+      return j + gstride >= e && ((((j - a) >> lgs) & 1) == 0);
+    };
+    // Fewer beads than threads: `parts` threads per bead, each with a run of the
+    // moved beads
+    const int cap = A.shape.term_cap, lim = min(nthr - nthr / 4, cap / 8);
+    struct Split {
+      int rest, part, parts, most, y;
+      bool put, last;
+      float4 pj;
+    };
+    // quotients of small integers: the half keeps them off the roundings
+    auto quotient = [](int a, int b) { return __float2int_rd(((float)a + 0.5f) * fast_rcp((float)b)); };
+    auto split = [&](bool kh, int x, int rest) {
+      Split S;
+      S.rest = rest;
+      S.part = quotient(tid, rest);
+      S.parts = quotient(nthr, rest);
+      S.most = quotient(cap, rest) & ~7;  // moved beads per round
+      const int j = bead_at(x + tid - S.part * rest, S.y, S.put);
+      S.pj = s_beads[j];
+      S.last = !kh && !CUT && odd_last(j);
+      return S;
+    };
+    const int xk = crowd || skip ? 0 : places(ncb), xe = places(N);
+    // Where that is all there is to the residue pairs (two short chains) it is
+    // worked out, and the beads are fetched, beside the trial positions, which
+    // a few warps are busy with: for 76 + 24 residues 900 to 450 cycles between
+    // them and the first pair, 2.96 to 2.79 us a step with the counters of this
+    // path on a warp of their own
+    const bool ahead = !spread && xk > 0 && xk <= lim;
+    const Split S0 = split(true, 0, max(xk, 1));
     {
       QuatProducts qp{};
       if (rot) qp = quat_products(r.q[0], r.q[1], r.q[2], r.q[3]);
@@ -994,41 +1052,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (!skip) {
       const PackedBox PB = packed_box(box, invbox);
       const float cut2 = s_tab[(kNT - 1) * kNT].z;
-      // bead at place x of the list of beads, the place y of its sum, and whether
-      // it counts. With one virtual CTA the list leaves the molecule out; else
-      // it holds this CTA's beads, the molecule's masked
-      auto bead_at = [&](int x, int& y, bool& counts) {
-        int j;
-        if (!CLUSTER || spread) {
-          j = x < m0 ? x : x + n;
-          y = j;
-          counts = true;
-        } else {
-          y = x;
-          j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
-          counts = (unsigned)(j - m0) >= (unsigned)n;
-        }
-        return j;
-      };
-      // places of the list below bead e
-      auto places = [&](int e) {
-        if (!CLUSTER || spread) return e <= m0 ? e : max(m0, e - n);
-        return ((e >> lgs) << lgv) + min(max((e & gmask) - vrank * vthr, 0), vthr);
-      };
       auto put_sum = [&](int y, float a) {
         if (spread)
           for (int k = 0; k < csize; ++k)
             cooperative_groups::this_cluster().map_shared_rank(s_aj, k)[y] = a;
         else
           s_aj[y] = a;
-      };
-      // is crowder pair j the odd one of its virtual thread's last pass (see
-      // wall_term)? Alone in a pass: a one-residue chain's pairs, and the
-      // chain beads a moved crowder meets
-      auto odd_last = [&](int j) {
-        if (n == 1 || j < ncb) return true;
-        const int a = j < m0 ? ncb : max(m0 + n, ncb), e = j < m0 ? m0 : N;
-        return j + gstride >= e && ((((j - a) >> lgs) & 1) == 0);
       };
       auto run_class = [&](auto kh, int x, int end) {
         constexpr bool KH = decltype(kh)::value;
@@ -1064,33 +1093,29 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
           for (int q = 0; q < NJ; ++q)
             if (put[q]) put_sum(y[q], a[q]);
         };
-        const int cap = A.shape.term_cap;
-        // two beads per lane while that keeps most threads at work, then one;
-        // what is left, fewer beads than threads, is split by terms
-        while (end - x > nthr + nthr / 2) {
-          if (x + warp * 32 + nthr < end)
-            whole(std::true_type{});
-          else
-            whole(std::false_type{});
-          x += 2 * nthr;
+        Split S = S0;
+        if (!KH || !ahead) {
+          // two beads per lane while that keeps most threads at work, then one;
+          // what is left, fewer beads than threads, is split by terms
+          while (end - x > nthr + nthr / 2) {
+            if (x + warp * 32 + nthr < end)
+              whole(std::true_type{});
+            else
+              whole(std::false_type{});
+            x += 2 * nthr;
+          }
+          while (end - x > lim) {
+            if (x + warp * 32 < end) whole(std::false_type{});
+            x += nthr;
+          }
+          if (end > x) S = split(KH, x, end - x);
         }
-        while (end - x > min(nthr - nthr / 4, cap / 8)) {
-          if (x + warp * 32 < end) whole(std::false_type{});
-          x += nthr;
-        }
-        // fewer beads than threads: `parts` threads per bead, each with a run of
-        // the moved beads, leave the terms, and one adds them in order
-        const int rest = end - x;
-        if (rest > 0) {
-          // quotients of small integers: the half keeps them off the roundings
-          auto quotient = [](int a, int b) { return __float2int_rd(((float)a + 0.5f) * fast_rcp((float)b)); };
-          const int part = quotient(tid, rest), parts = quotient(nthr, rest);
-          int y;
-          bool put;
-          const int j = bead_at(x + tid - part * rest, y, put);
-          const float4 pj = s_beads[j];
-          const bool last = !KH && !CUT && odd_last(j);
-          const int most = (cap / rest) & ~7;  // moved beads per round
+        // the parts' threads leave the terms, and one adds them in order
+        const int rest = S.rest;
+        if (end > x) {
+          const int part = S.part, parts = S.parts, most = S.most;
+          const float4 pj = S.pj;
+          const bool last = S.last;
           float a = 0.0f;
           for (int k0 = 0; k0 < n; k0 += most) {
             const int nk = min(most, n - k0);
@@ -1124,12 +1149,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
             }
             __syncthreads();
           }
-          if (tid < rest && put) put_sum(y, a);
+          if (tid < rest && S.put) put_sum(S.y, a);
         }
       };
-      const int xk = crowd ? 0 : places(ncb), xe = places(N);
-      run_class(std::true_type{}, 0, xk);
-      run_class(std::false_type{}, xk, xe);
+      if (xk > 0) run_class(std::true_type{}, 0, xk);
+      if (xe > xk) run_class(std::false_type{}, xk, xe);
     }
     if (spread)  // every a_j
       cluster_barrier();
@@ -1198,7 +1222,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       my_quat[2] = out[2];
       my_quat[3] = out[3];
     }
-    if (tid == 0) {
+    if (tid == 96) {  // warps 0 to 2 have installs, the rotation, the energies
       if (acc && !rot) cent[r.m] = make_float4(c_new.x, c_new.y, c_new.z, 0.0f);
       n_neg += acc == 1;
       n_boltz += acc == 2;
@@ -1242,12 +1266,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       A.n_samples[inst] += n_samp;
       A.n_bound[inst] += n_bnd;
     }
-    if (tid == 0) {
-      A.acc_neg[inst] += n_neg;
-      A.acc_boltz[inst] += n_boltz;
-      A.rej[inst] += n_rej;
-      A.evals_kh[inst] += ev_kh;
-      A.evals_crowd[inst] += ev_crowd;
+    if (tid == 0 || tid == 96) {  // the groups' counts, the other steps'
+      atomicAdd(&A.acc_neg[inst], n_neg);
+      atomicAdd(&A.acc_boltz[inst], n_boltz);
+      atomicAdd(&A.rej[inst], n_rej);
+      atomicAdd(&A.evals_kh[inst], ev_kh);
+      atomicAdd(&A.evals_crowd[inst], ev_crowd);
     }
   }
   __syncthreads();  // shared memory is reused by the next instance
