@@ -440,7 +440,8 @@ def main():
 
     # per timed step: ctrl_set_kernel (remc_run) + the graph's proposal_kernel,
     # block_cost_kernel and rank_kernel (work order by proposal cost, single
-    # CTAs per replica), sweep_kernel, exchange_kernel and ctrl_advance_kernel
+    # CTAs per replica), sweep_kernel (a second one where costly systems run on
+    # clusters beside the queue), exchange_kernel and ctrl_advance_kernel
     gpu_launches = args.steps * (3 + eng.work_order()[1])
     if rank == 0:
         line = {

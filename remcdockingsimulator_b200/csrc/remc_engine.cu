@@ -11,12 +11,16 @@
 // mol_base(s) + k*M_s.
 //
 // Kernels:
-//   sweep_kernel       one CTA per replica-instance, persistent over a whole
-//                      sweep of n_steps Metropolis steps; the instance's beads
-//                      and molecule centres stay resident in shared memory, each
-//                      step is proposal -> trial positions -> FP32 pair dE with
-//                      FP64 reduction -> Metropolis (Replica::MCSearch,
-//                      Replica.cpp:368-478, with dE in place of the full E).
+//   sweep_kernel       (remc_sweep.cuh) one CTA, or a cluster of them, per
+//                      replica-instance, persistent over a whole sweep of
+//                      n_steps Metropolis steps; the instance's beads and
+//                      molecule centres stay resident in shared memory.
+//                      Groups of one-bead moves, or one chain move: trial
+//                      positions -> FP32 pair dE, FP64 sums -> Metropolis
+//                      (Replica::MCSearch, Replica.cpp:368-478, with dE in
+//                      place of the full E).
+//   state_scan_kernel, state_pack_kernel  check an upload and decide each
+//                      system's minimum-image fold, then lay it out.
 //   energy_tile_kernel persistent grid over (instance, i-tile, j-tile) work
 //                      items of the upper triangle; per-item FP64 partials in a
 //                      scratch array, reduced per instance in fixed order by
@@ -1635,8 +1639,9 @@ int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
 // A cluster barrier with its remote stores costs some 1,500 cycles a pass, the
 // pairs of a chain step some 0.6 cycles each on one SM: a quarter of them per
 // CTA saves more from about 4,000 pairs on. Two chains of 76 and 24 residues
-// (1,824 pairs): 3.62 ms per 1000 steps spread, 3.15 not; 129 + 57 + 201
-// residues and 233 crowders (63,000): 0.80 ms spread, 1.17 not.
+// (1,824 pairs): 3.62 ms per 1000 steps spread, 3.15 not (now 2.79); 129 + 57 +
+// 201 residues and 233 turning crowders (63,000): 0.80 ms spread, 1.17 not (now
+// 0.66, groups running over the turns).
 constexpr double kSpreadPairs = 4096.0;
 
 // Add to a shape what fits in shared memory beside it without taking CTAs off

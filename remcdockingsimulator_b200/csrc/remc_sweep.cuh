@@ -21,7 +21,7 @@ struct SysDev {
   int crowd_type;     // the one bead type of every crowder, or -1 (none or mixed)
   // 1: every bead pair is within 1.5 box lengths on each axis, for the state
   // uploaded last and every state the sweep can reach from it (set on the
-  // device by fold_flag_kernel at each upload; the sweep then folds the
+  // device by state_pack_kernel at each upload; the sweep then folds the
   // minimum image)
   int fold_mi;
 };
