@@ -1645,7 +1645,9 @@ int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
 constexpr double kSpreadPairs = 4096.0;
 
 // Add to a shape what fits in shared memory beside it without taking CTAs off
-// the SM, and find how many CTAs an SM, and clusters the GPU, hold.
+// the SM, and find how many CTAs an SM, and clusters the GPU, hold. The second
+// is a query of some 1.1 ms; clusters of up to four CTAs that each fit an SM,
+// chosen here and not by the caller, go without it (null).
 int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* clusters) {
   if (allow_smem(h, shape.csize > 1, !shape.beads_in_smem)) return REMC_ERR_CUDA;
   const SweepFn fn = sweep_fn(h, shape.csize > 1, !shape.beads_in_smem);
@@ -1670,8 +1672,8 @@ int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* cl
   for (int cap = 4096; cap >= 1024 && !add(&SweepShape::term_cap, cap); cap /= 2) {
   }
   if (shape.beads_in_smem) add(&SweepShape::rel_in_smem, 1);
-  *clusters = 0;
-  if (shape.csize > 1) {
+  if (clusters) *clusters = 0;
+  if (clusters && shape.csize > 1) {
     // the cluster must be schedulable: csize CTAs of this size in one GPC
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -1766,12 +1768,11 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
       SweepShape wide = base_shape(h, threads, mol_in_smem, c, beads_in_smem);
       wide.vsize = 1;
       wide.aj_in_smem = 1;
-      int n = 0, k = 0;
-      if (SweepSmem::make(wide).total > (size_t)h->max_dyn_smem || fit_sweep(h, wide, block, &n, &k))
+      int n = 0;
+      if (SweepSmem::make(wide).total > (size_t)h->max_dyn_smem || fit_sweep(h, wide, block, &n, nullptr))
         continue;
       shape = wide;
       per_sm = n;
-      clusters = k;
       break;
     }
   }
@@ -1783,8 +1784,8 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
   apart.aj_in_smem = 1;
   if (shape.csize == 1 && beads_in_smem && SweepSmem::make(apart).total <= (size_t)h->max_dyn_smem) {
     choose_apart(h, per_sm * h->num_sms);
-    int n = 0, k = 0;
-    if (h->n_apart && (fit_sweep(h, apart, block, &n, &k) || ensure_sweep_scratch(h, apart))) {
+    int n = 0;
+    if (h->n_apart && (fit_sweep(h, apart, block, &n, nullptr) || ensure_sweep_scratch(h, apart))) {
       h->n_apart = 0;
       h->apart_from = INFINITY;
     }
