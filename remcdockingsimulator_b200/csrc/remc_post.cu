@@ -102,50 +102,64 @@ __device__ __forceinline__ float dist3(const float* a, const float* b) {
 }
 
 constexpr int kDrmsThreads = 256;
-constexpr int kDrmsFrames = 4;  // frames a CTA takes against one evaluation of the reference
+constexpr int kDrmsFrames = 4;  // frames a CTA takes against one evaluation of the reference: a float4
 
 // Per (group of kDrmsFrames frames, part of the i beads): a warp takes one bead
 // i at a time and its lanes the beads j of later molecules, side by side. A
 // reference distance (two with REVERSE) serves all frames of the group. The
-// frames sit in shared memory by coordinate (SHARED; frames too large for it
-// are read from global memory). Bound by the square roots: 4 chains of 150, 500
-// frames, both orders, ran 378 us with one CTA per frame, a thread per bead i
-// and both distances evaluated per frame and pair.
+// frames sit in shared memory by coordinate, the four values of a bead in one
+// load (SHARED; frames too large for it are read from global memory). Bound by
+// issue slots, the square roots' among them: 4 chains of 150, 500 frames, both
+// orders, ran 378 us with one CTA per frame, a thread per bead i and both
+// distances evaluated per frame and pair, 229 us in two CTAs per SM with a load
+// per frame and a last round of 33 CTAs, 165 us now.
 // out[frame][part]: sums; counts[frame][part]: native, recovered, binding pairs.
 struct DrmsOut {
   double a, b;
   unsigned long long native, recovered, binding;
 };
 template <bool REVERSE, bool SHARED>
-__global__ void __launch_bounds__(kDrmsThreads) drms_kernel(
+__global__ void __launch_bounds__(kDrmsThreads, 3) drms_kernel(
     const float* __restrict__ frames, int n_frames, const float* __restrict__ ref,
     const int* __restrict__ ms, const int* __restrict__ mol_of, int n_beads, float native_cut,
     float recovered_cut, DrmsOut* __restrict__ out) {
-  extern __shared__ float s_x[];  // [frame][coordinate][bead]
+  extern __shared__ float4 s_x[];  // [coordinate][bead], the frames side by side
   __shared__ DrmsOut s_out[kDrmsThreads / 32][kDrmsFrames];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f0 = blockIdx.x * kDrmsFrames, nf = min(kDrmsFrames, n_frames - f0);
   const float* x = frames + (size_t)f0 * n_beads * 3;
   if (SHARED) {
-    for (int e = tid; e < nf * n_beads * 3; e += kDrmsThreads) {
-      const int bead = e / 3, f = bead / n_beads;
-      s_x[(3 * f + e - 3 * bead) * n_beads + bead - f * n_beads] = x[e];
+    for (int e = tid; e < n_beads * 3; e += kDrmsThreads) {
+      const int bead = e / 3;
+      float v[kDrmsFrames];
+#pragma unroll
+      for (int f = 0; f < kDrmsFrames; ++f)  // past the last frame: repeated, not written out
+        v[f] = x[(size_t)min(f, nf - 1) * n_beads * 3 + e];
+      s_x[(e - 3 * bead) * n_beads + bead] = make_float4(v[0], v[1], v[2], v[3]);
     }
     __syncthreads();
   }
-  auto at = [&](int f, int c, int bead) {
-    return SHARED ? s_x[(3 * f + c) * n_beads + bead] : x[((size_t)f * n_beads + bead) * 3 + c];
+  // coordinate c of a bead in every frame
+  auto at = [&](int c, int bead, float (&v)[kDrmsFrames]) {
+    if (SHARED) {
+      const float4 q = s_x[c * n_beads + bead];
+      v[0] = q.x;
+      v[1] = q.y;
+      v[2] = q.z;
+      v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int f = 0; f < kDrmsFrames; ++f) v[f] = x[((size_t)min(f, nf - 1) * n_beads + bead) * 3 + c];
+    }
   };
   double sa[kDrmsFrames] = {}, sb[kDrmsFrames] = {};
   unsigned cn = 0, cr[kDrmsFrames] = {}, cb[kDrmsFrames] = {};
   const int warps = (kDrmsThreads / 32) * gridDim.y;
   for (int i = blockIdx.y * (kDrmsThreads / 32) + warp; i < n_beads; i += warps) {
     const int I = mol_of[i], li = i - ms[I];
-    float xi[kDrmsFrames][3];
+    float xi[3][kDrmsFrames];
 #pragma unroll
-    for (int f = 0; f < kDrmsFrames; ++f)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) xi[f][c] = at(min(f, nf - 1), c, i);
+    for (int c = 0; c < 3; ++c) at(c, i, xi[c]);
     for (int j = ms[I + 1] + lane; j < n_beads; j += 32) {  // beads of molecules J > I
       const float de = dist3(ref + 3 * i, ref + 3 * j);
       float dr = 0.0f;
@@ -156,11 +170,13 @@ __global__ void __launch_bounds__(kDrmsThreads) drms_kernel(
       }
       const bool near = de < native_cut;
       cn += near;
+      float xj[3][kDrmsFrames];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) at(c, j, xj[c]);
 #pragma unroll
       for (int f = 0; f < kDrmsFrames; ++f) {
-        const int g = min(f, nf - 1);  // past the last frame: repeated, not written out
-        const float ds = length3(__fsub_rn(xi[f][0], at(g, 0, j)), __fsub_rn(xi[f][1], at(g, 1, j)),
-                                 __fsub_rn(xi[f][2], at(g, 2, j)));
+        const float ds = length3(__fsub_rn(xi[0][f], xj[0][f]), __fsub_rn(xi[1][f], xj[1][f]),
+                                 __fsub_rn(xi[2][f], xj[2][f]));
         sa[f] += (double)fabsf(__fsub_rn(ds, de));
         if (REVERSE) sb[f] += (double)fabsf(__fsub_rn(ds, dr));
         cr[f] += near && ds < recovered_cut;
@@ -196,6 +212,25 @@ __global__ void __launch_bounds__(kDrmsThreads) drms_kernel(
     }
     out[(size_t)(f0 + tid) * gridDim.y + blockIdx.y] = t;
   }
+}
+
+// Parts a group of frames is split into, of `most`: the fewest rounds of `slots`
+// resident CTAs, weighed by a part's length, which is the group's pairs over
+// the parts plus the loading of the frames, some 1.5 pairs a bead. About four
+// CTAs per SM instead, 625 of them for 125 groups, left a third round on 296
+// slots with 33.
+int drms_parts(int groups, int slots, int most, double beads_per_pair) {
+  int best = 1;
+  double least = INFINITY;
+  for (int p = 1; p <= std::min(most, 64); ++p) {
+    const long long rounds = ((long long)groups * p + slots - 1) / slots;
+    const double t = (double)rounds * (1.0 / p + 1.5 * beads_per_pair);
+    if (t < least) {
+      least = t;
+      best = p;
+    }
+  }
+  return best;
 }
 
 // One slab of device memory for a call, from a pool per device that keeps up to
@@ -335,17 +370,25 @@ int remc_post_drms(const float* frames, int n_frames, const float* ref, const in
     for (int b = mol_start[m]; b < mol_start[m + 1]; ++b) mol_of[b] = m;
     n_pairs += (double)(mol_start[m + 1] - mol_start[m]) * (double)(nb - mol_start[m + 1]);
   }
-  // groups of frames, and parts of the i beads where the groups are too few for
-  // the GPU (about two CTAs per SM)
+  // groups of frames, each in parts of the i beads
   int dev = 0, sms = 148, smem_max = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const int groups = (n_frames + kDrmsFrames - 1) / kDrmsFrames;
   const int most = std::max(1, nb / (2 * (kDrmsThreads / 32)));
-  const int parts = std::max(1, std::min(most, (4 * sms + groups - 1) / groups));
   const size_t smem = sizeof(float) * 3 * (size_t)nb * kDrmsFrames;
   const bool shared = smem + 4096 <= (size_t)smem_max;
+  auto kernel = reverse ? (shared ? drms_kernel<true, true> : drms_kernel<true, false>)
+                        : (shared ? drms_kernel<false, true> : drms_kernel<false, false>);
+  cudaError_t e = cudaSuccess;
+  if (shared && smem > 48 * 1024)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 0;
+  if (e != cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                              &per_sm, kernel, kDrmsThreads, shared ? smem : 0) != cudaSuccess)
+    per_sm = 1;
+  const int parts = drms_parts(groups, std::max(1, per_sm) * sms, most, nb / n_pairs);
   const size_t n_out = (size_t)n_frames * parts;
   Slab B;
   const size_t o_x = B.take(sizeof(float) * 3 * (size_t)nb * n_frames), o_ref = B.take(sizeof(float) * 3 * nb),
@@ -359,11 +402,6 @@ int remc_post_drms(const float* frames, int n_frames, const float* ref, const in
       (rc = copy_in(d_mol, (const int*)mol_of.data(), (size_t)nb)) ||
       (rc = copy_in(d_x, frames, 3 * (size_t)nb * n_frames)))
     return rc;
-  auto kernel = reverse ? (shared ? drms_kernel<true, true> : drms_kernel<true, false>)
-                        : (shared ? drms_kernel<false, true> : drms_kernel<false, false>);
-  cudaError_t e = cudaSuccess;
-  if (shared && smem > 48 * 1024)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   std::vector<DrmsOut> out(n_out);
   if (e == cudaSuccess) {
     kernel<<<dim3(groups, parts), kDrmsThreads, shared ? smem : 0>>>(

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("lengths,frames", [
-    ([1, 1], 1), ([1, 40, 3], 3), ([33, 31], 4), ([20] * 5, 5), ([150] * 4, 9),
+    ([1, 1], 1), ([1, 40, 3], 3), ([33, 31], 4), ([20] * 5, 5), ([150] * 4, 9), ([30] * 3, 303),
     ([2500, 2400], 2),  # 4 frames of 4900 beads exceed a CTA's shared memory
 ])
 def test_drms_shapes(built_lib, lengths, frames):
