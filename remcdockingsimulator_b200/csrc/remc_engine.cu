@@ -1139,69 +1139,6 @@ __global__ void __launch_bounds__(128) deps_kernel(double* __restrict__ G, doubl
   }
 }
 
-// dE/dlambda alone (the sensitivities' call): only residue pairs depend on
-// lambda, so the tiles are those of the chains. The per-type-pair sums are the
-// adjoint kernel's, term for term and tile for tile (lane L takes eight beads j
-// in the order q ^ r there, which is kept), and go into dE/dlambda at the end of
-// the tile. Grid (tile pair, instance); a crowded system of 500 beads has one
-// tile pair instead of ten: 31 us a call for 32 replicas, from 99 with the whole
-// adjoint, a copy of the sums and a loop on the host.
-__global__ void __launch_bounds__(kTile) lambda_tile_kernel(
-    const SysDev* __restrict__ sys, const int* __restrict__ inst_sys,
-    const float4* __restrict__ pos, const float4* __restrict__ tab,
-    const int* __restrict__ mol_start, float c_lj, double* __restrict__ dl, int inst0,
-    const __grid_constant__ ContactTable T) {
-  const int inst = inst0 + blockIdx.y, tid = threadIdx.x, lane = tid & 31;
-  const SysDev S = sys[inst_sys[inst]];
-  const int ncb = S.n_chain_beads, nt = (ncb + kTile - 1) / kTile;
-  int ti = 0, tj = blockIdx.x;  // row ti holds nt - ti tiles
-  while (ti < nt && tj >= nt - ti) tj -= nt - ti++;
-  if (ti >= nt) return;
-  tj += ti;
-  __shared__ float4 s_j[kTile];
-  __shared__ float2 s_tab[kNumAmino * kNumAmino];  // sigma^2, repulsive-branch threshold
-  __shared__ float s_G[kNumAmino * kNumAmino];
-  const size_t base = S.bead_base + (size_t)(inst - S.inst0) * S.n_beads;
-  const int j0 = tj * kTile, jn = min(kTile, ncb - j0);
-  if (tid < jn) s_j[tid] = pos[base + j0 + tid];
-  for (int k = tid; k < kNumAmino * kNumAmino; k += kTile) {
-    const float4 t = tab[(k / kNumAmino) * kNT + k % kNumAmino];
-    s_tab[k] = make_float2(t.y, t.z);
-    s_G[k] = 0.0f;
-  }
-  __syncthreads();
-  const int i = ti * kTile + tid;
-  {
-    const float4 pi = i < ncb ? pos[base + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int ta = bead_type(pi.w);
-    // later beads of other molecules: from the own molecule's end on
-    const int lo = i < ncb ? max(mol_start[S.mstart_off + bead_mol(pi.w) + 1], i + 1) - j0 : jn;
-    const int r = (lane >> 2) & 7;
-    for (int jg = ti == tj ? (tid & ~31) : 0; jg < jn; jg += 8)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int j = jg + (q ^ r);
-        if (j < lo || j >= jn) continue;
-        const float4 pj = s_j[j];
-        const int e = ta * kNumAmino + bead_type(pj.w);
-        const float2 t = s_tab[e];
-        const float r2 = pair_r2(pi, pj, S.box, S.invbox);
-        const float rinv = fast_rsqrt(r2);
-        const float s2 = t.x * (rinv * rinv);
-        const float s6 = s2 * s2 * s2;
-        float dg = 4.0f * fmaf(-s6, s6, s6);
-        dg = r2 < t.y ? 2.0f - dg : dg;
-        atomicAdd(&s_G[e], dg * c_lj);
-      }
-  }
-  __syncthreads();
-  double acc = 0.0;
-  for (int k = tid; k < kNumAmino * kNumAmino; k += kTile)
-    acc += (double)s_G[k] * ((double)T.m[k] - (double)T.e0);
-  acc = warp_sum(acc);
-  if (lane == 0 && acc != 0.0) atomicAdd(&dl[inst], acc);
-}
-
 // ------------------------------------------------------------------ exchange
 __global__ void exchange_kernel(const SysDev* __restrict__ sys, const float* __restrict__ ladder,
                                 const double* __restrict__ energy, int* __restrict__ temp_idx,
@@ -2701,23 +2638,8 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   ContactTable table;
   memcpy(table.m, h->pair_table, sizeof(table.m));
   table.e0 = h->params.e0;
-  const float c_lj = (float)((double)h->params.lj_cf * (double)h->params.kbt_cf);
   int rc = REMC_OK;
   if (!h->d_dl && (rc = dev_alloc(&h->d_dl, h->n_inst))) return rc;
-  if (dE_dlambda && !forces && !mol_force_torque && !dE_dxi && !dE_deps && !energy) {
-    int nt = 0;
-    for (const SysDev& S : h->h_sys) nt = std::max(nt, (S.n_chain_beads + kTile - 1) / kTile);
-    REMC_CUDA_TRY(cudaMemsetAsync(h->d_dl, 0, sizeof(double) * h->n_inst, h->stream));
-    if (nt > 0) {
-      for (int g = 0; g < h->n_inst; g += 32768) {  // grid rows are limited
-        const int n = std::min(32768, h->n_inst - g);
-        lambda_tile_kernel<<<dim3(nt * (nt + 1) / 2, n), kTile, 0, h->stream>>>(
-            h->d_sys, h->d_inst_sys, h->d_pos, h->d_tab, h->d_mol_start, c_lj, h->d_dl, g, table);
-        REMC_CUDA_TRY(cudaGetLastError());
-      }
-    }
-    return fetch(h, {{dE_dlambda, h->d_dl, sizeof(double) * h->n_inst}});
-  }
   if (!h->d_adj_acc) {
     // forces first, every part on a 256-byte boundary
     auto up256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -2741,7 +2663,7 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   AdjConsts C;
   C.inv_xi = 1.0f / h->params.debye_length;
   C.inv_xi2 = C.inv_xi * C.inv_xi;
-  C.c_lj = c_lj;
+  C.c_lj = (float)((double)h->params.lj_cf * (double)h->params.kbt_cf);
   const bool cut = h->params.crowder_cutoff > 0.0f;
   auto adj = h->params.crowder_mode ? (cut ? adjoint_tile_kernel<true, true>
                                            : adjoint_tile_kernel<true, false>)
@@ -2757,9 +2679,11 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
                                      h->d_items_by_cost, h->n_items, h->d_adj_queue, h->d_forces,
                                      h->d_G, h->d_dxi, h->d_eadj, consts_of(h), C);
   REMC_CUDA_TRY(cudaGetLastError());
-  molecule_force_torque_kernel<<<dim3(h->n_inst, (h->mmax + 127) / 128), 128, 0, h->stream>>>(
-      h->d_sys, h->d_inst_sys, h->d_mol_start, h->d_rel, h->d_forces, h->d_mft);
-  REMC_CUDA_TRY(cudaGetLastError());
+  if (mol_force_torque) {
+    molecule_force_torque_kernel<<<dim3(h->n_inst, (h->mmax + 127) / 128), 128, 0, h->stream>>>(
+        h->d_sys, h->d_inst_sys, h->d_mol_start, h->d_rel, h->d_forces, h->d_mft);
+    REMC_CUDA_TRY(cudaGetLastError());
+  }
   if (dE_deps || dE_dlambda) {
     deps_kernel<<<h->n_inst, 128, 0, h->stream>>>(h->d_G, h->d_dl, table);
     REMC_CUDA_TRY(cudaGetLastError());
@@ -2770,21 +2694,12 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
   if (mol_force_torque)
     REMC_CUDA_TRY(cudaMemcpyAsync(mol_force_torque, h->d_mft, sizeof(double) * 6 * h->total_mols,
                                   cudaMemcpyDeviceToHost, h->stream));
-  if (dE_dxi)
-    REMC_CUDA_TRY(cudaMemcpyAsync(dE_dxi, h->d_dxi, sizeof(double) * h->n_inst,
-                                  cudaMemcpyDeviceToHost, h->stream));
-  if (energy)
-    REMC_CUDA_TRY(cudaMemcpyAsync(energy, h->d_eadj, sizeof(double) * h->n_inst,
-                                  cudaMemcpyDeviceToHost, h->stream));
-  if (dE_dlambda)
-    REMC_CUDA_TRY(cudaMemcpyAsync(dE_dlambda, h->d_dl, sizeof(double) * h->n_inst,
-                                  cudaMemcpyDeviceToHost, h->stream));
   if (dE_deps)
     REMC_CUDA_TRY(cudaMemcpyAsync(dE_deps, h->d_G,
                                   sizeof(double) * kNumAmino * kNumAmino * (size_t)h->n_inst,
                                   cudaMemcpyDeviceToHost, h->stream));
-  REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  return REMC_OK;
+  const size_t n = sizeof(double) * h->n_inst;
+  return fetch(h, {{dE_dxi, h->d_dxi, n}, {energy, h->d_eadj, n}, {dE_dlambda, h->d_dl, n}});
 }
 
 int remc_get_noncrowder_energies(remc_handle* h, double* out) {
