@@ -755,8 +755,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   };
 
   // Records up to `avail` can be read, up to `filled` are requested. The
-  // records before this pass are read by nobody any more (the last pass ended
-  // with a barrier), and a ring half that lies before it is requested anew.
+  // records before this pass are read by nobody any more (a pass takes what it
+  // needs of its own before the barrier that ends it), and a ring half that
+  // lies before it is requested anew.
   int avail = min(kRing, n_steps), filled = avail;
   int parity = 0;      // buffer of this pass's sums (clusters alternate)
   bool alone = false;  // the next step's sum does not split: taken like a chain step
@@ -874,9 +875,14 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       const StepRec& mine = s_ring[(s + (lane < gsize ? lane : 0)) & (kRing - 1)];
       const unsigned group_movers = movers;
       const bool turns = warp == nwarps - 1 && crank == 0 && lane < gsize && my_rot;
-      double4 quat = make_double4(0.0, 0.0, 0.0, 0.0);
+      double4 quat = make_double4(0.0, 0.0, 0.0, 0.0), turn = quat;
       double* const my_quat = A.quat + 4 * (size_t)(mol_off + my_m);
-      if (turns) quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
+      bool accepts = false;
+      if (turns) {  // the record too: behind the closing barrier its place may be refilled
+        quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
+        turn = make_double4(mine.q[0], mine.q[1], mine.q[2], mine.q[3]);
+        accepts = mine.thr > 0.0;
+      }
       if (warp == 0) {
         double hi = 0.0, lo = 0.0;
         const bool moves = lane < gsize && !my_rot;
@@ -937,9 +943,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       __syncthreads();  // the group's installs and s_done
       const int done = s_done;
       pending = 2 + (pending & 1 ^ 1);  // the sums just left for warp 2, the next buffer
-      if (turns && lane < done && mine.thr > 0.0) {
+      if (accepts && lane < done) {
         double out[4];
-        quat_mul(mine.q[0], mine.q[1], mine.q[2], mine.q[3], quat.x, quat.y, quat.z, quat.w, out);
+        quat_mul(turn.x, turn.y, turn.z, turn.w, quat.x, quat.y, quat.z, quat.w, out);
         my_quat[0] = out[0];
         my_quat[1] = out[1];
         my_quat[2] = out[2];

@@ -1,0 +1,36 @@
+"""Crowders that turn, over many refills of the ring of proposals: accumulated
+rotations equal one launch per step bit for bit, in single CTAs, in replicas
+spread over clusters of two and four, and beside costly systems, also where a
+sampling chunk cuts the groups short."""
+import numpy as np
+import pytest
+
+from test_gpu_sweep_groups import _sweep, _system
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("chains,R,every", [
+    ([20, 24], 12, 0), ([20, 24], 12, 20),      # a CTA per replica
+    ([90, 100], 5, 0), ([90, 100], 5, 20),      # clusters of four
+    ([90, 100], 40, 0), ([90, 100], 40, 7),     # clusters of two
+])
+def test_turns_over_many_refills(built_lib, chains, R, every):
+    from remcdockingsimulator_b200.engine import make_params
+    s = _system(2, chains, 70, 6.0, 170.0, turn=True)
+    got = _sweep([s], R, make_params(), 800, 9, 128, every=every)
+    want = _sweep([s], R, make_params(), 800, 9, 128, plain=True)
+    for a, b in zip(got[1], want[1]):
+        assert np.array_equal(a, b)
+    if every:
+        assert np.all(got[3][0] == 800 // every)
+
+
+def test_turns_beside_costly_systems(built_lib):
+    from remcdockingsimulator_b200.engine import make_params
+    systems = [_system(k, [20, 25 + k], 10 + 10 * k, 6.0, 120.0, turn=True) for k in range(7)]
+    systems.insert(3, _system(11, [250, 260, 240, 230], 80, 6.0, 300.0, turn=True))
+    got = _sweep(systems, 20, make_params(), 160, 9, 128)
+    want = _sweep(systems, 20, make_params(), 160, 9, 128, plain=True)
+    for a, b in zip(got[1], want[1]):
+        assert np.array_equal(a, b)
