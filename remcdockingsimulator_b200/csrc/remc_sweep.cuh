@@ -101,6 +101,41 @@ __host__ __device__ inline int held_sums(const SweepShape& s) {
   return local_beads(s) * (s.csize > s.vsize ? 2 : 1);
 }
 
+// The beads whose sums a chain step takes, as one CTA goes through them, for a
+// moved molecule of n beads from m0 on. Of a replica of one virtual CTA they are
+// all but the molecule's, and a sum's place is its bead; else those of the CTA's
+// own virtual threads, the molecule's masked, and places count them.
+struct BeadList {
+  int m0, n;
+  bool own;            // the CTA's own virtual threads' beads
+  int vthr, lgv, lgs;  // virtual threads of a CTA, logarithms of it and of the replica's
+  int vrank;
+  // the bead at position x of the list, the place y of its sum, does it count
+  __host__ __device__ int bead(int x, int& y, bool& counts) const {
+    if (!own) {
+      const int j = x < m0 ? x : x + n;
+      y = j;
+      counts = true;
+      return j;
+    }
+    const int j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
+    y = x;
+    counts = (unsigned)(j - m0) >= (unsigned)n;
+    return j;
+  }
+  // positions of the list below bead e: all that bead() may be asked for
+  __host__ __device__ int places(int e) const {
+    if (!own) return e <= m0 ? e : (m0 > e - n ? m0 : e - n);
+    const int rest = (e & ((1 << lgs) - 1)) - vrank * vthr;
+    return ((e >> lgs) << lgv) + (rest < 0 ? 0 : rest > vthr ? vthr : rest);
+  }
+};
+// Are a step's xk residue pairs' beads fetched ahead? Only of a list that has
+// some, and one the threads have split among them.
+__host__ __device__ inline bool fetch_ahead(bool spread, int xk, int lim) {
+  return !spread && xk > 0 && xk <= lim;
+}
+
 struct SweepArgs {
   const SysDev* sys;
   const int* inst_sys;
@@ -970,27 +1005,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (turns) quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
     const float4 c_old = cent[r.m];
     const float4 c_new = rot ? c_old : translated(c_old, r.t);
-    // bead at place x of the list of beads, the place y of its sum, and whether
-    // it counts. With one virtual CTA the list leaves the molecule out; else
-    // it holds this CTA's beads, the molecule's masked
-    auto bead_at = [&](int x, int& y, bool& counts) {
-      int j;
-      if (!CLUSTER || spread) {
-        j = x < m0 ? x : x + n;
-        y = j;
-        counts = true;
-      } else {
-        y = x;
-        j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
-        counts = (unsigned)(j - m0) >= (unsigned)n;
-      }
-      return j;
-    };
-    // places of the list below bead e
-    auto places = [&](int e) {
-      if (!CLUSTER || spread) return e <= m0 ? e : max(m0, e - n);
-      return ((e >> lgs) << lgv) + min(max((e & gmask) - vrank * vthr, 0), vthr);
-    };
+    const BeadList list{m0, n, CLUSTER && !spread, vthr, lgv, lgs, vrank};
     // is crowder pair j the odd one of its virtual thread's last pass (see
     // wall_term)? Alone in a pass: a one-residue chain's pairs, and the
     // chain beads a moved crowder meets
@@ -1015,19 +1030,20 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       S.part = quotient(tid, rest);
       S.parts = quotient(nthr, rest);
       S.most = quotient(cap, rest) & ~7;  // moved beads per round
-      const int j = bead_at(x + tid - S.part * rest, S.y, S.put);
+      const int j = list.bead(x + tid - S.part * rest, S.y, S.put);
       S.pj = s_beads[j];
       S.last = !kh && !CUT && odd_last(j);
       return S;
     };
-    const int xk = crowd || skip ? 0 : places(ncb), xe = places(N);
+    const int xk = crowd || skip ? 0 : list.places(ncb), xe = list.places(N);
     // Where that is all there is to the residue pairs (two short chains) it is
     // worked out, and the beads are fetched, beside the trial positions, which
     // a few warps are busy with: for 76 + 24 residues 900 to 450 cycles between
     // them and the first pair, 2.96 to 2.79 us a step with the counters of this
     // path on a warp of their own
-    const bool ahead = !spread && xk > 0 && xk <= lim;
-    const Split S0 = split(true, 0, max(xk, 1));
+    const bool ahead = fetch_ahead(spread, xk, lim);
+    Split S0{};
+    if (ahead) S0 = split(true, 0, xk);
     {
       QuatProducts qp{};
       if (rot) qp = quat_products(r.q[0], r.q[1], r.q[2], r.q[3]);
@@ -1083,7 +1099,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
 #pragma unroll
           for (int q = 0; q < NJ; ++q) {
             const int at = x + tid + q * nthr;
-            const int j = bead_at(min(at, end - 1), y[q], put[q]);
+            const int j = list.bead(min(at, end - 1), y[q], put[q]);
             put[q] = put[q] && at < end;
             pj[q] = s_beads[j];
             last[q] = !KH && !CUT && odd_last(j);
