@@ -279,14 +279,19 @@ __global__ void __launch_bounds__(256) state_scan_kernel(
       float w = s_v[tid][0];
       for (int q = 1; q < 8; ++q) w = fmaxf(w, s_v[tid][q]);
       part[(size_t)tid * n_cta + inst * gridDim.y + blockIdx.y] = w;
+    }
+    __syncthreads();
+    // one thread's fences on both sides of the count, between barriers, order
+    // what all threads of a CTA wrote or reported (part, bad) before what all
+    // threads of the last one read
+    if (tid == 0) {
+      __threadfence();
+      s_last = atomicAdd(&res->done, 1u) == (unsigned)n_cta - 2u;  // counts from ~0
       __threadfence();
     }
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&res->done, 1u) == (unsigned)n_cta - 2u;  // counts from ~0
-    __syncthreads();
     if (!s_last) return;
   }
-  __threadfence();
   // the last CTA: systems by warp, or all warps on one system's columns at a time
   const bool together = n_sys < 8;
   const int step = together ? 1 : 8;
