@@ -20,9 +20,9 @@ def test_lambda_alone_sums_as_the_adjoint(built_lib, chains, crowders, box):
             only.append(eng.dE_dlambda())
     full, only = np.array(full), np.array(only)
     # the sums are atomics' (their order is not fixed), so calls scatter: the
-    # two means differ by some sqrt(2/16) of one call's deviation; 4 of them
-    # is beyond chance. FP64 sums over the type pairs add 1e-12
+    # two means differ by some sqrt(2/16) of one call's deviation; four times
+    # that is beyond chance. FP64 sums over the type pairs add 1e-12
     mean = full.mean(axis=0)
     size = np.linalg.norm(mean)
     scatter = np.sqrt(np.mean(np.sum((full - mean) ** 2, axis=1)))
-    assert np.linalg.norm(only.mean(axis=0) - mean) <= 4.0 * scatter + 1e-12 * size
+    assert np.linalg.norm(only.mean(axis=0) - mean) <= 4.0 * np.sqrt(2.0 / 16.0) * scatter + 1e-12 * size
