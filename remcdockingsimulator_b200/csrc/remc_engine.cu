@@ -2263,8 +2263,10 @@ int remc_set_params(remc_handle* h, const remc_params* p) {
     return set_error(REMC_ERR_INVALID, "bad parameters");
   h->params = *p;
   h->config_gen++;  // a captured graph holds the old constants and kernel
+  // the parameters may name other kernels: of the schedule, of costly systems
+  // apart (clusters, beads in shared memory), of one launch per step
   if (allow_smem(h, h->sweep_shape.csize > 1, !h->beads_in_smem) ||
-      allow_smem(h, false, !h->beads_in_smem))
+      (h->n_apart && allow_smem(h, true, false)) || allow_smem(h, false, !h->beads_in_smem))
     return REMC_ERR_CUDA;
   if (h->tables_set) return build_tables(h);
   return REMC_OK;
