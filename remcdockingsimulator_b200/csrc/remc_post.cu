@@ -382,8 +382,15 @@ int remc_post_drms(const float* frames, int n_frames, const float* ref, const in
   auto kernel = reverse ? (shared ? drms_kernel<true, true> : drms_kernel<true, false>)
                         : (shared ? drms_kernel<false, true> : drms_kernel<false, false>);
   cudaError_t e = cudaSuccess;
-  if (shared && smem > 48 * 1024)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (shared && smem > 48 * 1024) {
+    // always the same limit, whatever this call needs: another host thread's
+    // call may be between setting it and its launch
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, kernel);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               smem_max - (int)attr.sharedSizeBytes);
+  }
   int per_sm = 0;
   if (e != cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                               &per_sm, kernel, kDrmsThreads, shared ? smem : 0) != cudaSuccess)
