@@ -76,7 +76,8 @@ int CUDA_memcpy_to_host_async(void* destination, void* source, int mem_size,
  * Each (device, stream) has its own partial-sum buffer, kept until exit and
  * grown only after the stream's queued work has finished: energies queued on
  * different streams (the reference gives every replica thread its own,
- * main.cpp:924-954) may run concurrently, from any host threads. */
+ * main.cpp:924-954) may run concurrently, from any host threads. For
+ * cudaStreamPerThread each host thread has its own. */
 void CUDA_EonDevice_async(float4* residuePositions, float4* residueMeta, int* residueCount,
                           int* moleculePositions, int* moleculeCount, float* LJPotentials,
                           float* device_result, int resultSize, int blockSize, int datasetSize,

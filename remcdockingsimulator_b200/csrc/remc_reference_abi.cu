@@ -50,13 +50,51 @@ remc_params g_params;
 // lookup until its last launch (and, on the synchronous path, its result
 // copy) is enqueued, so calls on one stream take their turns in stream order,
 // and calls on different streams or host threads never share partials.
+// cudaStreamPerThread is one handle for another stream in every host thread:
+// each thread has a slot of its own for it, which goes to a later thread once
+// its last call has ended on the GPU, so there are as many as threads at a time.
 struct ScratchSlot {
   std::mutex mu;
   double* ptr = nullptr;
   size_t cap = 0;
+  cudaEvent_t used = nullptr;  // behind the last call, of a thread's slot
 };
 std::mutex g_slots_mutex;
 std::map<std::pair<int, cudaStream_t>, std::unique_ptr<ScratchSlot>> g_slots;
+// slots of threads that have ended, by device (never destroyed: threads may end late)
+std::multimap<int, ScratchSlot*>& idle_slots() {
+  static auto* idle = new std::multimap<int, ScratchSlot*>();
+  return *idle;
+}
+struct ThreadSlots {
+  std::map<int, ScratchSlot*> by_device;
+  ~ThreadSlots() {
+    std::lock_guard<std::mutex> g(g_slots_mutex);
+    for (const auto& s : by_device)
+      if (s.second) idle_slots().insert(s);
+  }
+};
+thread_local ThreadSlots t_slots;
+
+// This thread's slot for cudaStreamPerThread; null on failure.
+ScratchSlot* thread_slot(int dev) {
+  ScratchSlot*& mine = t_slots.by_device[dev];
+  if (mine) return mine;
+  std::lock_guard<std::mutex> g(g_slots_mutex);
+  const auto range = idle_slots().equal_range(dev);
+  for (auto it = range.first; it != range.second; ++it) {
+    if (cudaEventQuery(it->second->used) == cudaSuccess) {
+      mine = it->second;
+      idle_slots().erase(it);
+      return mine;
+    }
+    cudaGetLastError();  // not ready is no error
+  }
+  std::unique_ptr<ScratchSlot> made(new ScratchSlot());
+  if (cudaEventCreateWithFlags(&made->used, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+  mine = made.release();
+  return mine;
+}
 
 void set_status(int code, const char* what, cudaError_t e = cudaSuccess) {
   g_status = code;
@@ -103,6 +141,14 @@ struct RefItems {
 // for larger structures, whose items are many anyway.
 constexpr int kRefChunk = 32;
 constexpr int kRefSmallTiles = 48;
+// Counters of finished items, one per number of items: the word of the items'
+// counter, or -1 for structures beyond some 112,000 beads, whose call of
+// milliseconds adds its partials in a second launch. A call that another one
+// overlaps (a captured call replayed on another stream) shares its partials
+// and may get a wrong sum, but leaves no counter off for later calls: each
+// word goes round from zero to zero with every call's items, and only calls
+// of as many items count in it.
+constexpr int kRefCounters = 1024;
 RefItems ref_items(int P, bool chunks = true) {
   RefItems it;
   it.P = P;
@@ -111,6 +157,11 @@ RefItems ref_items(int P, bool chunks = true) {
   it.per = kRefTile / jt;
   it.C = (P + jt - 1) / jt;
   return it;
+}
+
+int ref_counter(const RefItems& it) {
+  const int word = it.per > 1 ? it.C : kRefSmallTiles * (kRefTile / kRefChunk - 1) + it.C;
+  return word < kRefCounters ? word : -1;
 }
 
 // Fixed-order sum of n partials by one CTA; thread 0 has it.
@@ -143,7 +194,7 @@ __device__ void put_total(double total, const RefTotal& R) {
 }
 
 // One item per CTA (chunk blockIdx.x, tile blockIdx.y). With `done` the last CTA
-// to finish adds the partials, in a fixed order, and sets the counter back.
+// to finish adds the partials, in a fixed order; the counter is then at zero.
 template <int JT>
 __global__ void __launch_bounds__(kRefTile) ref_energy_tiles(
     const float4* __restrict__ pos, const float4* __restrict__ meta,
@@ -208,35 +259,38 @@ __global__ void __launch_bounds__(kRefTile) ref_energy_tiles(
     for (int w = 0; w < kRefTile / 32; ++w) t += s_red[w];
     partials[it.offset(ti) + c - it.first(ti)] = t;
     if (done) {
+      const unsigned last = (unsigned)it.count() - 1u;
       __threadfence();
-      s_last = atomicAdd(done, 1u) == (unsigned)it.count() - 1u;
+      s_last = atomicInc(done, last) == last;
+      __threadfence();
     }
   }
   if (!done) return;
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
   const double sum = sum_partials<kRefTile>(partials, it.count(), s_red);
   put_total(sum, total);
-  if (tid == 0) *done = 0u;
 }
 
-// Fixed-order sum of n partials (one CTA), for the call whose calls may overlap
-// and so cannot share a counter.
+// Fixed-order sum of n partials (one CTA), for calls without a counter.
 __global__ void ref_energy_sum(const double* __restrict__ partials, int n, RefTotal total) {
   __shared__ double s[256];
   put_total(sum_partials<256>(partials, n, s), total);
 }
 
-// Launch the items; `done` (may be null): the last CTA adds the partials.
-cudaError_t launch_ref_items(const float4* pos, const float4* meta, const float* table,
-                             const RefItems& it, double* partials, const RefConsts& C,
-                             unsigned* done, const RefTotal& total, cudaStream_t stream) {
+// Launch the items and the sum of their partials: by the last CTA with `done`,
+// by a launch of its own without.
+cudaError_t launch_energy(const float4* pos, const float4* meta, const float* table,
+                          const RefItems& it, double* partials, const RefConsts& C,
+                          unsigned* done, const RefTotal& total, cudaStream_t stream) {
   const dim3 grid(it.C, it.T);
   if (it.per == 1)
     ref_energy_tiles<kRefTile><<<grid, kRefTile, 0, stream>>>(pos, meta, table, it, partials, C, done, total);
   else
     ref_energy_tiles<kRefChunk><<<grid, kRefTile, 0, stream>>>(pos, meta, table, it, partials, C, done, total);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || done) return e;
+  ref_energy_sum<<<1, 256, 0, stream>>>(partials, it.count(), total);
   return cudaGetLastError();
 }
 
@@ -283,6 +337,23 @@ __global__ void translate_center_kernel(float4* center, const float4* t) {
   center->z += v.z;
 }
 
+// Sets a new buffer's counters to zero before the stream's next work: on the
+// stream, or, where that is being captured (it would happen in the graph only),
+// now.
+bool clear_counters(double* scratch, cudaStream_t stream) {
+  const size_t bytes = sizeof(unsigned) * kRefCounters;
+  cudaStreamCaptureStatus capture;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return false;
+  if (capture == cudaStreamCaptureStatusNone)
+    return cudaMemsetAsync(scratch, 0, bytes, stream) == cudaSuccess;
+  cudaStream_t s;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return false;
+  const bool ok = cudaMemsetAsync(scratch, 0, bytes, s) == cudaSuccess &&
+                  cudaStreamSynchronize(s) == cudaSuccess;
+  cudaStreamDestroy(s);
+  return ok;
+}
+
 // The scratch buffer of (current device, stream), locked by `lock`, holding
 // at least n doubles. Growing it first waits for the work already queued on
 // the stream (the only work that can still read the old buffer) and frees it.
@@ -291,7 +362,10 @@ double* stream_scratch(cudaStream_t stream, size_t n, std::unique_lock<std::mute
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return nullptr;
   ScratchSlot* slot;
-  {
+  if (stream == cudaStreamPerThread) {
+    slot = thread_slot(dev);
+    if (!slot) return nullptr;
+  } else {
     std::lock_guard<std::mutex> g(g_slots_mutex);
     std::unique_ptr<ScratchSlot>& p = g_slots[std::make_pair(dev, stream)];
     if (!p) p.reset(new ScratchSlot());
@@ -307,7 +381,7 @@ double* stream_scratch(cudaStream_t stream, size_t n, std::unique_lock<std::mute
     }
     const size_t cap = std::max<size_t>(n, 4096);
     if (cudaMalloc(&slot->ptr, cap * sizeof(double)) != cudaSuccess ||
-        cudaMemsetAsync(slot->ptr, 0, sizeof(double), stream) != cudaSuccess) {
+        !clear_counters(slot->ptr, stream)) {
       cudaFree(slot->ptr);
       slot->ptr = nullptr;
       return nullptr;
@@ -345,19 +419,22 @@ bool energy_args_ok(const float4* pos, const float4* meta, const float* table, i
   return true;
 }
 
-// Doubles of scratch for an energy call: the counter of finished items (zero
-// between calls, which take turns on their stream), the total, the partials.
-size_t ref_scratch(int P) { return (size_t)ref_items(P).count() + 2; }
+// A call's scratch, in doubles: the counters of finished items (zero between
+// calls, which take turns on their stream), the total, the partials.
+constexpr size_t kRefTotal = sizeof(unsigned) * kRefCounters / sizeof(double);
+size_t ref_scratch(int P) { return kRefTotal + 1 + (size_t)ref_items(P).count(); }
 
-// Enqueue the energy of P beads on `stream`; the total goes to scratch[1] and,
-// optionally, to the reference's per-block grid.
+// Enqueue the energy of P beads on `stream`; the total goes to scratch[kRefTotal]
+// and, optionally, to the reference's per-block grid.
 int enqueue_energy(const float4* pos, const float4* meta, const float* table, int P,
                    double* scratch, float* grid_out, int grid_n, cudaStream_t stream) {
-  RefTotal total{scratch + 1, grid_out, grid_n, 1.0f};
+  RefTotal total{scratch + kRefTotal, grid_out, grid_n, 1.0f};
   const RefConsts C = make_consts(&total.unscale);
+  const RefItems it = ref_items(P);
+  const int word = ref_counter(it);
   const cudaError_t e =
-      launch_ref_items(pos, meta, table, ref_items(P), scratch + 2, C,
-                       reinterpret_cast<unsigned*>(scratch), total, stream);
+      launch_energy(pos, meta, table, it, scratch + kRefTotal + 1, C,
+                    word < 0 ? nullptr : reinterpret_cast<unsigned*>(scratch) + word, total, stream);
   if (e != cudaSuccess) {
     set_status(REMC_ERR_CUDA, "energy kernel launch", e);
     return REMC_ERR_CUDA;
@@ -466,7 +543,7 @@ void CUDA_EonDevice(float4* pos, float4* meta, int* residueCount, int* moleculeP
     return;
   }
   if (enqueue_energy(pos, meta, table, datasetSize, scratch, nullptr, 0, 0) != REMC_OK) return;
-  cudaError_t e = cudaMemcpy(result, scratch + 1, sizeof(double), cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemcpy(result, scratch + kRefTotal, sizeof(double), cudaMemcpyDeviceToHost);
   set_status(e == cudaSuccess ? REMC_OK : REMC_ERR_CUDA, "result copy", e);
 }
 
@@ -497,6 +574,15 @@ void CUDA_EonDevice_async(float4* pos, float4* meta, int* residueCount, int* mol
   if (enqueue_energy(pos, meta, table, datasetSize, scratch, device_result,
                      resultSize * resultSize, stream) != REMC_OK)
     return;
+  if (stream == cudaStreamPerThread) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaEventRecord(thread_slot(dev)->used, stream);
+    if (e != cudaSuccess) {
+      set_status(REMC_ERR_CUDA, "event record", e);
+      return;
+    }
+  }
   set_status(REMC_OK, "");
 }
 
@@ -599,15 +685,10 @@ int CUDA_EonDevice_noalloc(const float4* pos, const float4* meta, const float* L
   }
   // every item writes its partial before the sum reads it: no clearing needed
   const RefConsts C = make_consts();
-  e = launch_ref_items(pos, meta, table, it, scratch, C, nullptr, RefTotal{}, stream);
+  e = launch_energy(pos, meta, table, it, scratch, C, nullptr, RefTotal{d_result, nullptr, 0, 1.0f},
+                    stream);
   if (e != cudaSuccess) {
     set_status(REMC_ERR_CUDA, "energy kernel launch", e);
-    return REMC_ERR_CUDA;
-  }
-  ref_energy_sum<<<1, 256, 0, stream>>>(scratch, it.count(), RefTotal{d_result, nullptr, 0, 1.0f});
-  e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_status(REMC_ERR_CUDA, "energy sum launch", e);
     return REMC_ERR_CUDA;
   }
   set_status(REMC_OK, "");
