@@ -947,8 +947,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
           }
           left_movers &= left_movers - 1u;
         }
-        // a sum that did not split (NaN) ends the group before its step, which
-        // is then taken by itself
+        // a sum that did not split (NaN) ends the group before its step
         const unsigned broke = __ballot_sync(full, lane < gsize && isnan(dE));
         const int done = broke ? __ffs(broke) - 1 : gsize;
         const bool acc = lane < done && dE < thr;
@@ -986,10 +985,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
         my_quat[2] = out[2];
         my_quat[3] = out[3];
       }
-      alone = done < gsize;
+      // a group's first step is evaluated against its own state: if its sum does
+      // not split there, it goes alone; a later one first begins a new group
+      alone = done == 0;
       s += done;
       if (to_sample > 0 && (to_sample -= done) == 0) sample(s);
-      if ((warp == 0 || alone) && s < n_steps) look(s, avail, to_sample);
+      if ((warp == 0 || done < gsize) && s < n_steps) look(s, avail, to_sample);
       continue;
     }
 
