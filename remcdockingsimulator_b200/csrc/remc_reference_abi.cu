@@ -235,10 +235,9 @@ __global__ void __launch_bounds__(kRefTile) ref_energy_tiles(
       const float i6 = rinv2 * rinv2 * rinv2;
       if (use && r2 < C.cutoff2) lj += 46656.0f * i6;  // (6/r)^6
     } else if (use) {
-      // rint of the index, as an integer, without a conversion
-      int idx = __float_as_int(__fadd_rn(__fadd_rn(row, mj.x), 12582912.0f)) - 0x4b400000;
-      idx = min(max(idx, 0), 399);
-      const float eps = s_eps[idx];
+      // rint of the index in [0, 399] (no number: 0), without a conversion
+      const float in = fminf(fmaxf(__fadd_rn(row, mj.x), 0.0f), 399.0f);
+      const float eps = s_eps[__float_as_int(__fadd_rn(in, 12582912.0f)) - 0x4b400000];
       const float sig = (mi.z + mj.z) * 0.5f;
       const float sig2 = sig * sig;
       const float s2 = sig2 * rinv2;

@@ -71,3 +71,33 @@ def test_reference_call_sizes(built_lib, n_beads):
     assert L.CUDA_EonDevice_noalloc(p(dp.data_ptr()), p(dm.data_ptr()), p(dt.data_ptr()), P,
                                     p(out.data_ptr()), p(torch.cuda.current_stream().cuda_stream)) == 0
     assert abs(out.item() - sync.value) <= 1e-12 * abs(sync.value)
+
+
+@pytest.mark.parametrize("ti,tj,entry", [
+    (3.0, 7.0, 67), (19.0, 19.0, 399), (float("nan"), 4.0, 0), (2.0, float("nan"), 0),
+    (-3.0, 4.0, 0), (-2e7, 4.0, 0), (25.0, 0.0, 399), (2e9, 0.0, 399), (float("inf"), 0.0, 399),
+    (float("-inf"), 5.0, 0), (1.0, 0.4, 20), (1.0, 0.6, 21),
+])
+def test_contact_table_entry(built_lib, ti, tj, entry):
+    """The entry of a pair is the nearest of 20 ti + tj in the table, the first
+    one where that is no number: a table of zeros but for it gives the energy
+    that a table of that value throughout gives."""
+    import torch
+    from remcdockingsimulator_b200.reference_abi import abi
+    L, p = abi(), C.c_void_p
+    pos = torch.tensor([[10.0, 10.0, 10.0, 0.0], [15.0, 10.0, 10.0, 1.0]], device="cuda")
+    meta = torch.tensor([[ti, 0.0, 6.0, 0.0], [tj, 0.0, 6.0, 0.0]], device="cuda")
+    L.CUDA_setBoxDimension(100.0)
+
+    def energy(table):
+        out = C.c_double(0.0)
+        L.CUDA_EonDevice(p(pos.data_ptr()), p(meta.data_ptr()), None, None, None,
+                         p(table.data_ptr()), C.byref(out), 32, 2, 0)
+        assert L.remc_reference_abi_status() == 0
+        return out.value
+
+    one = torch.zeros(400, device="cuda")
+    one[entry] = -5.0
+    torch.cuda.synchronize()
+    want = energy(torch.full((400,), -5.0, device="cuda"))
+    assert energy(one) == want and want != energy(torch.zeros(400, device="cuda"))
