@@ -1406,7 +1406,11 @@ void free_all(remc_handle* h) {
 
 int build_tables(remc_handle* h) {
   const remc_params& P = h->params;
-  std::vector<float4> tab(kNT * kNT);
+  // the table, and behind it the bits of the residue types whose row has a
+  // Debye-Hueckel term (found by every warp of the sweep from the table, entry
+  // by entry, they had taken 4 us of a launch)
+  std::vector<float4> tab(kNT * kNT + 1);
+  unsigned charged = 0;
   const float c_lj = (float)((double)P.lj_cf * (double)P.kbt_cf);
   const float c_dh = (float)((double)P.dh_const * (double)P.kbt_cf);
   const float two_third = 1.2599210498948732f;  // 2^(1/3): (2^(1/6) sigma)^2 = 2^(1/3) sigma^2
@@ -1422,6 +1426,7 @@ int build_tables(remc_handle* h) {
         t.y = sig * sig;
         t.z = eps > 0.0f ? sig * sig * two_third : -1.0f;
         t.w = h->charge[a] * h->charge[b] * c_dh;
+        if (t.w != 0.0f) charged |= 1u << a;
       } else {
         double A;
         if (P.crowder_mode == 0) {
@@ -1439,6 +1444,7 @@ int build_tables(remc_handle* h) {
       tab[a * kNT + b] = t;
     }
   }
+  memcpy(&tab[kNT * kNT].x, &charged, sizeof(charged));
   REMC_CUDA_TRY(cudaMemcpyAsync(h->d_tab, tab.data(), sizeof(float4) * tab.size(),
                                 cudaMemcpyHostToDevice, h->stream));
   REMC_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -2142,7 +2148,7 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   if (!rc) rc = dev_alloc(&h->d_mol_start, h->h_mol_start.size());
   if (!rc) rc = dev_alloc(&h->d_mol_role, h->h_mol_role.size());
   if (!rc) rc = dev_alloc(&h->d_mrole_off, h->n_sys);
-  if (!rc) rc = dev_alloc(&h->d_tab, (size_t)kNT * kNT);
+  if (!rc) rc = dev_alloc(&h->d_tab, (size_t)kNT * kNT + 1);
   if (!rc) rc = dev_alloc(&h->d_energy, h->n_inst);
   if (!rc) rc = dev_alloc(&h->d_temp_idx, h->n_inst);
   if (!rc) rc = dev_alloc(&h->d_slot_of_temp, h->n_inst);

@@ -622,14 +622,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
   float4* const cent = A.shape.mol_in_smem ? reinterpret_cast<float4*>(smem_raw + L.centres)
                                            : A.centre + mol_off;
 
-  // residue types with charges, by the type table
-  unsigned charged;
-  {
-    bool any = false;
-    if (lane < kNumAmino)
-      for (int t = 0; t < kNumAmino; ++t) any = any || A.tab[lane * kNT + t].w != 0.0f;
-    charged = __ballot_sync(full, any);
-  }
+  // residue types with charges: the word behind the type table
+  const unsigned charged = __float_as_uint(A.tab[kNT * kNT].x);
 
   // ---- prologue: make the instance resident in shared memory
   for (int i = tid; i < kNT * kNT; i += nthr) s_tab[i] = A.tab[i];
