@@ -101,33 +101,35 @@ __host__ __device__ inline int held_sums(const SweepShape& s) {
   return local_beads(s) * (s.csize > s.vsize ? 2 : 1);
 }
 
-// The beads whose sums a chain step takes, as one CTA goes through them, for a
-// moved molecule of n beads from m0 on. Of a replica of one virtual CTA they are
-// all but the molecule's, and a sum's place is its bead; else those of the CTA's
-// own virtual threads, the molecule's masked, and places count them.
+// The beads whose sums a chain step takes, as one CTA goes through them: all but
+// the moved molecule's n from m0 on, of a replica of one virtual CTA; else those
+// of them that belong to the CTA's own virtual threads. A sum's place counts the
+// CTA's beads, the molecule's among them.
 struct BeadList {
-  int m0, n;
   bool own;            // the CTA's own virtual threads' beads
   int vthr, lgv, lgs;  // virtual threads of a CTA, logarithms of it and of the replica's
   int vrank;
-  // the bead at position x of the list, the place y of its sum, does it count
-  __host__ __device__ int bead(int x, int& y, bool& counts) const {
-    if (!own) {
-      const int j = x < m0 ? x : x + n;
-      y = j;
-      counts = true;
-      return j;
-    }
-    const int j = ((x >> lgv) << lgs) + vrank * vthr + (x & (vthr - 1));
-    y = x;
-    counts = (unsigned)(j - m0) >= (unsigned)n;
-    return j;
+  int gap, skip;       // place and number of the molecule's beads
+  __host__ __device__ BeadList(int m0, int n, bool own_, int vthr_, int lgv_, int lgs_, int vrank_)
+      : own(own_), vthr(vthr_), lgv(lgv_), lgs(lgs_), vrank(vrank_) {
+    gap = place(m0);
+    skip = place(m0 + n) - gap;
   }
-  // positions of the list below bead e: all that bead() may be asked for
-  __host__ __device__ int places(int e) const {
-    if (!own) return e <= m0 ? e : (m0 > e - n ? m0 : e - n);
+  // the CTA's beads below bead e
+  __host__ __device__ int place(int e) const {
+    if (!own) return e;
     const int rest = (e & ((1 << lgs) - 1)) - vrank * vthr;
     return ((e >> lgs) << lgv) + (rest < 0 ? 0 : rest > vthr ? vthr : rest);
+  }
+  // positions of the list below bead e: all that bead() may be asked for
+  __host__ __device__ int positions(int e) const {
+    const int p = place(e);
+    return p <= gap ? p : (gap > p - skip ? gap : p - skip);
+  }
+  // the bead at position x of the list, and the place y of its sum
+  __host__ __device__ int bead(int x, int& y) const {
+    y = x < gap ? x : x + skip;
+    return own ? ((y >> lgv) << lgs) + vrank * vthr + (y & (vthr - 1)) : y;
   }
 };
 // Are a step's xk residue pairs' beads fetched ahead? Only of a list that has
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     if (turns) quat = make_double4(my_quat[0], my_quat[1], my_quat[2], my_quat[3]);
     const float4 c_old = cent[r.m];
     const float4 c_new = rot ? c_old : translated(c_old, r.t);
-    const BeadList list{m0, n, CLUSTER && !spread, vthr, lgv, lgs, vrank};
+    const BeadList list(m0, n, CLUSTER && !spread, vthr, lgv, lgs, vrank);
     // is crowder pair j the odd one of its virtual thread's last pass (see
     // wall_term)? Alone in a pass: a one-residue chain's pairs, and the
     // chain beads a moved crowder meets
@@ -1014,7 +1016,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
     const int cap = A.shape.term_cap, lim = min(nthr - nthr / 4, cap / 8);
     struct Split {
       int rest, part, parts, most, y;
-      bool put, last;
+      bool last;
       float4 pj;
     };
     // quotients of small integers: the half keeps them off the roundings
@@ -1025,12 +1027,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       S.part = quotient(tid, rest);
       S.parts = quotient(nthr, rest);
       S.most = quotient(cap, rest) & ~7;  // moved beads per round
-      const int j = list.bead(x + tid - S.part * rest, S.y, S.put);
+      const int j = list.bead(x + tid - S.part * rest, S.y);
       S.pj = s_beads[j];
       S.last = !kh && !CUT && odd_last(j);
       return S;
     };
-    const int xk = crowd || skip ? 0 : list.places(ncb), xe = list.places(N);
+    const int xk = crowd || skip ? 0 : list.positions(ncb), xe = list.positions(N);
     // Where that is all there is to the residue pairs (two short chains) it is
     // worked out, and the beads are fetched, beside the trial positions, which
     // a few warps are busy with: for 76 + 24 residues 900 to 450 cycles between
@@ -1094,8 +1096,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
 #pragma unroll
           for (int q = 0; q < NJ; ++q) {
             const int at = x + tid + q * nthr;
-            const int j = list.bead(min(at, end - 1), y[q], put[q]);
-            put[q] = put[q] && at < end;
+            const int j = list.bead(min(at, end - 1), y[q]);
+            put[q] = at < end;
             pj[q] = s_beads[j];
             last[q] = !KH && !CUT && odd_last(j);
             any_last = any_last || last[q];
@@ -1166,7 +1168,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
             }
             __syncthreads();
           }
-          if (tid < rest && S.put) put_sum(S.y, a);
+          if (tid < rest) put_sum(S.y, a);
         }
       };
       if (xk > 0) run_class(std::true_type{}, 0, xk);

@@ -29,30 +29,29 @@ int main() {
             const bool own = vsize > 1;
             std::vector<int> seen(N, 0);
             for (int r = 0; r < vsize; ++r) {
-              const BeadList list{m0, n, own, vthr, lg(vthr), lg(vthr * vsize), r};
-              const int end = list.places(N);
+              const BeadList list(m0, n, own, vthr, lg(vthr), lg(vthr * vsize), r);
+              const int end = list.positions(N);
               int before = -1, y;
-              bool counts;
               for (int x = 0; x < end; ++x) {
-                const int j = list.bead(x, y, counts);
-                if (j <= before || j >= N || y < 0 || y >= (own ? end : N)) return 1;
-                if (counts != !(j >= m0 && j < m0 + n)) return 2;
-                seen[j] += counts;
+                const int j = list.bead(x, y);
+                if (j <= before || j >= N || y < x || y >= list.place(N)) return 1;
+                if (j >= m0 && j < m0 + n) return 2;
+                ++seen[j];
                 before = j;
               }
               // the residue pairs' beads, fetched by every thread of the CTA
               for (int ncb : {0, 1, 44, N}) {
                 if (ncb > N) continue;
-                const int xk = list.places(ncb);
-                if (xk > list.places(N)) return 3;
+                const int xk = list.positions(ncb);
+                if (xk > list.positions(N)) return 3;
                 for (int spread = 0; spread < 2; ++spread) {
-                  if (!remc::fetch_ahead(spread, xk, nthr - nthr / 4)) {
-                    if (xk == 0 && list.bead(0, y, counts) >= N) ++outside;
+                  if (!remc::fetch_ahead(spread, xk, nthr / 2)) {
+                    if (xk == 0 && list.bead(0, y) >= N) ++outside;
                     continue;
                   }
                   if (xk < 1) return 4;
                   for (int tid = 0; tid < nthr; ++tid) {
-                    const int j = list.bead(tid - tid / xk * xk, y, counts);
+                    const int j = list.bead(tid - tid / xk * xk, y);
                     if (j < 0 || j >= N) return 5;
                     ++fetched;
                   }
