@@ -1011,9 +1011,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       const int a = j < m0 ? ncb : max(m0 + n, ncb), e = j < m0 ? m0 : N;
       return j + gstride >= e && ((((j - a) >> lgs) & 1) == 0);
     };
-    // Fewer beads than threads: `parts` threads per bead, each with a run of the
-    // moved beads
-    const int cap = A.shape.term_cap, lim = min(nthr - nthr / 4, cap / 8);
+    // At least two threads for every bead: `parts` threads per bead, each with a
+    // run of the moved beads. With one thread per bead the terms' way through
+    // shared memory, in rounds of a few moved beads, only costs: 300 beads on
+    // 512 threads 90,000 cycles a step split, 70,000 whole
+    const int cap = A.shape.term_cap, lim = min(nthr / 2, cap / 8);
     struct Split {
       int rest, part, parts, most, y;
       bool last;
