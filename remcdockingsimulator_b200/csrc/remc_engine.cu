@@ -38,8 +38,10 @@
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "remc_device.cuh"
@@ -1306,6 +1308,7 @@ struct remc_handle {
   // pinned host memory that kernels write: the error word of bounded waits, the
   // upload scan's report, energies
   unsigned char* h_pin = nullptr;
+  size_t pin_size = 0;
   int* pin_err = nullptr;
   ScanReport* pin_scan = nullptr;
   double* pin_energy = nullptr;
@@ -1383,7 +1386,56 @@ int dev_alloc(T** p, size_t n) {
   return REMC_OK;
 }
 
+// Pinned blocks of ended handles, for later ones of any thread and device: to
+// allocate one takes 1 to 3 ms and to free it 0.5, creating and ending a handle
+// for 500 beads by 32 replicas 3.4 without. Up to 1 MiB is kept, the rest freed.
+constexpr size_t kPinnedBlock = (size_t)64 << 10, kPinnedKeep = (size_t)1 << 20;
+struct PinnedPool {
+  std::mutex mu;
+  std::vector<std::pair<size_t, unsigned char*>> idle;
+  size_t kept = 0;
+};
+PinnedPool& pinned_pool() {
+  static auto* pool = new PinnedPool();  // never destroyed: handles may end late
+  return *pool;
+}
+
+// A block of at least `size` bytes, whose size it sets; null on failure.
+unsigned char* take_pinned(size_t& size) {
+  size = (size + kPinnedBlock - 1) / kPinnedBlock * kPinnedBlock;
+  PinnedPool& pool = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    for (auto& b : pool.idle)
+      if (b.first == size) {
+        unsigned char* p = b.second;
+        b = pool.idle.back();
+        pool.idle.pop_back();
+        pool.kept -= size;
+        return p;
+      }
+  }
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, size, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+  return static_cast<unsigned char*>(p);
+}
+
+// Gives a block back; nothing on the GPU may still use it.
+void give_pinned(unsigned char* p, size_t size) {
+  PinnedPool& pool = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    if (pool.kept + size <= kPinnedKeep) {
+      pool.idle.emplace_back(size, p);
+      pool.kept += size;
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 void free_all(remc_handle* h) {
+  if (h->stream) cudaStreamSynchronize(h->stream);
   void* ptrs[] = {h->d_sys,      h->d_inst_sys,  h->d_inst_list,  h->d_inst_cost,  h->d_inst_order,
                   h->d_pos,        h->d_rel,
                   h->d_centre,   h->d_quat,      h->d_mol_start,  h->d_tab,        h->d_energy,
@@ -1399,7 +1451,7 @@ void free_all(remc_handle* h) {
                   h->d_sweep_scratch, h->d_scan_part, h->d_scan, h->d_sys_cost};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  if (h->h_pin) cudaFreeHost(h->h_pin);
+  if (h->h_pin) give_pinned(h->h_pin, h->pin_size);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
@@ -2182,9 +2234,9 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
   if (!rc) {
     const size_t o_scan = 16, o_energy = (o_scan + sizeof(ScanReport) + sizeof(int) * h->n_sys + 15) & ~(size_t)15;
     const size_t o_fetch = (o_energy + sizeof(double) * h->n_inst + 15) & ~(size_t)15;
-    if (cudaHostAlloc((void**)&h->h_pin, o_fetch + 3 * (sizeof(double) * h->n_inst + 16),
-                      cudaHostAllocMapped) != cudaSuccess) {
-      h->h_pin = nullptr;
+    h->pin_size = o_fetch + 3 * (sizeof(double) * h->n_inst + 16);
+    h->h_pin = take_pinned(h->pin_size);
+    if (!h->h_pin) {
       rc = set_error(REMC_ERR_NOMEM, "pinned host memory");
     } else {
       h->pin_err = reinterpret_cast<int*>(h->h_pin);
@@ -2257,7 +2309,6 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
 
 int remc_destroy(remc_handle* h) {
   if (!h) return REMC_OK;
-  if (h->stream) cudaStreamSynchronize(h->stream);
   free_all(h);
   delete h;
   return REMC_OK;
