@@ -1738,6 +1738,45 @@ void choose_apart(remc_handle* h, int slots) {
   }
 }
 
+// Threads of a sweep CTA, for a schedule of `threads` virtual threads and `ctas`
+// CTAs in all. The kernel's registers fill an SM with 512 threads.
+//
+// With crowders two warps per virtual warp, 256 or 512: a group of 8 steps then
+// has whole warps or pairs of warps for every step. Without, chain steps only,
+// which all threads share: 512 where a step has pairs for them, 256 for less
+// (100 residues, 20 replicas, 1000 steps: 2.64 ms, 2.79 with 512).
+//
+// With more CTAs than SMs hold, those wait for whole rounds, and small steps,
+// which are latency, run as fast on fewer threads: half as many, down to 128,
+// where the systems are small. us for 100 steps, 128 / 256 / 512 threads (in
+// brackets 128 without groups and splits): 20 + 24 residues, 300 replicas 268 /
+// 444 / 685 (353); 100 residues, 1200 replicas 1197 / 1497 / 2482 (1851); 300 +
+// 300 residues, 150 replicas 6062 / 5359 / 7172 (6322); 44 residues and 100
+// crowders, 1200 replicas 304 / 328 / 533 (382); but 100 residues and 400
+// crowders, 600 replicas 243 / 212 / 312 (277).
+constexpr double kWidePairs = 16384.0, kHeavyPairs = 65536.0;
+constexpr int kSmallBeads = 192, kTinyBeads = 96;
+int sweep_block(const remc_handle* h, int threads, long long ctas) {
+  const double pairs = h->chain_step_pairs;
+  int block, least;
+  if (h->any_crowders) {
+    block = std::min(kSweepThreads, std::max(256, 2 * threads));
+    least = h->nmax <= kSmallBeads ? 128 : block;
+  } else {
+    block = pairs >= kWidePairs ? kSweepThreads : 256;
+    least = pairs < kHeavyPairs ? 128 : 256;
+  }
+  // up to half a round more of 256 threads where groups keep them busy: 104
+  // beads, 300 replicas 96 us in two rounds of 256, 102 in one of 128; 54 beads,
+  // 250 and 235
+  auto round = [&](int b) {
+    const long long n = (long long)h->num_sms * (kSweepThreads / b);
+    return h->any_crowders && b == 256 && h->nmax > kTinyBeads ? n + n / 2 : n;
+  };
+  while (block > least && ctas > round(block)) block /= 2;
+  return block;
+}
+
 // Set the sweep schedule: virtual threads per CTA (they fix the order of the
 // sums, see remc_sweep.cuh), where molecule data lives, CTAs per replica, and
 // whether the beads are resident in shared memory.
@@ -1752,13 +1791,21 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
     return set_error(REMC_ERR_INVALID,
                      "largest system needs %zu bytes of shared memory, device allows %d", least,
                      h->max_dyn_smem);
-  // Two warps per virtual warp: a group of 8 steps then has whole warps (128
-  // virtual threads) or pairs of warps (256) for every step. Systems without
-  // crowders have chain steps only, which all threads share: 512
-  const int block = h->any_crowders ? std::min(kSweepThreads, std::max(256, 2 * threads)) : kSweepThreads;
+  int block = sweep_block(h, threads, (long long)h->n_inst * csize);
   int per_sm = 0, clusters = 0;
   const int rc = fit_sweep(h, shape, block, &per_sm, &clusters);
   if (rc) return rc;
+  if (csize > 1 && clusters < h->n_inst && block > 256) {
+    // smaller CTAs where clusters of the larger would run the replicas in waves
+    SweepShape other = base_shape(h, threads, mol_in_smem, csize, beads_in_smem);
+    int n = 0, c = 0;
+    if (!fit_sweep(h, other, 256, &n, &c) && c > clusters) {
+      shape = other;
+      block = 256;
+      per_sm = n;
+      clusters = c;
+    }
+  }
   // Replicas fewer than the SMs: a replica of one virtual CTA spreads over a
   // cluster of up to four, each on its own SM, where its chain steps are long
   // enough (kSpreadPairs) for the cluster barrier they then take.

@@ -1182,30 +1182,28 @@ __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(const SweepArgs
       __syncthreads();
 
     // ---- virtual threads' sums, virtual warps' FP64 sums, one fixed tree
-    double d_all = 0.0, d_cc = 0.0;
-    if (!skip && tid < vthr) {
-      float acc_c = 0.0f, acc_o = 0.0f;
-      for (int j = vrank * vthr + tid, y = tid; j < N; j += gstride, y += vthr) {
-        if ((unsigned)(j - m0) < (unsigned)n) continue;
-        const float a = s_aj[y];
-        if (j < ncb && !crowd)
-          acc_c += a;
-        else
-          acc_o += a;
-      }
-      d_cc = (double)acc_c;
-      d_all = (double)acc_o;
-    }
-    if (warp < 8) {
-      // sums of d_all in lanes 0-15, of d_cc in 16-31, each in warp_sum's order;
-      // zero for virtual warps there are none of
+    // sums of residue and of crowder pairs, the first in lanes 16-31, the other
+    // in 0-15, each in warp_sum's order; zero for virtual warps there are none of
+    for (int w = warp; w < 8; w += nwarps) {
       double v = 0.0;
-      if (32 * warp < vthr) v = warp_sum_split(d_all, d_cc, lane);
+      if (32 * w < vthr) {
+        float acc_c = 0.0f, acc_o = 0.0f;
+        if (!skip)
+          for (int y = 32 * w + lane, j = vrank * vthr + y; j < N; j += gstride, y += vthr) {
+            if ((unsigned)(j - m0) < (unsigned)n) continue;
+            const float a = s_aj[y];
+            if (j < ncb && !crowd)
+              acc_c += a;
+            else
+              acc_o += a;
+          }
+        v = warp_sum_split((double)acc_o, (double)acc_c, lane);
+      }
       if ((lane & 15) == 0)
         for (int k = 0; k < vsize; ++k) {
           double* dst = sums;
           if (CLUSTER && !spread) dst = cooperative_groups::this_cluster().map_shared_rank(sums, k);
-          dst[16 * vrank + (lane >> 1) + warp] = v;
+          dst[16 * vrank + (lane >> 1) + w] = v;
         }
     }
     if (landing) cp_async_wait_all();

@@ -5,7 +5,7 @@ sampling chunk cuts the groups short."""
 import numpy as np
 import pytest
 
-from test_gpu_sweep_groups import _sweep, _system
+from test_gpu_sweep_groups import _check, _sweep, _system
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +34,15 @@ def test_turns_beside_costly_systems(built_lib):
     want = _sweep(systems, 20, make_params(), 160, 9, 128, plain=True)
     for a, b in zip(got[1], want[1]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("chains,crowders,turn", [
+    ([20, 24], 0, False), ([90, 90], 0, False), ([20, 24], 12, False), ([20, 24], 40, True)])
+@pytest.mark.parametrize("R,threads", [(160, 128), (340, 128), (340, 256)])
+def test_cta_sizes(built_lib, chains, crowders, turn, R, threads):
+    """More replicas than fit at once: CTAs of 512, 256 and 128 threads, fewer
+    threads than virtual threads among them, against the oracle's trajectory and
+    one launch per step."""
+    from remcdockingsimulator_b200.engine import make_params
+    s = _system(7, chains, crowders, 6.0, 140.0, turn=turn)
+    _check([s], R, make_params(), 40, threads)
