@@ -1644,11 +1644,31 @@ int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
 // 0.66, groups running over the turns).
 constexpr double kSpreadPairs = 4096.0;
 
+// Clusters of a fitted shape that the GPU holds at once: csize CTAs of this size
+// in one GPC each. A query of some 1.1 ms. 0 if none.
+int cluster_room(const remc_handle* h, const SweepShape& shape, int block) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = shape.csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(shape.csize);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = SweepSmem::make(shape).total;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int room = 0;
+  if (cudaOccupancyMaxActiveClusters(&room, sweep_fn(h, true, !shape.beads_in_smem), &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return room;
+}
+
 // Add to a shape what fits in shared memory beside it without taking CTAs off
-// the SM, and find how many CTAs an SM, and clusters the GPU, hold. The second
-// is a query of some 1.1 ms; clusters of up to four CTAs that each fit an SM,
-// chosen here and not by the caller, go without it (null).
-int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* clusters) {
+// the SM, and find how many CTAs an SM holds.
+int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm) {
   if (allow_smem(h, shape.csize > 1, !shape.beads_in_smem)) return REMC_ERR_CUDA;
   const SweepFn fn = sweep_fn(h, shape.csize > 1, !shape.beads_in_smem);
   auto resident = [&](const SweepShape& p) {
@@ -1672,25 +1692,6 @@ int fit_sweep(remc_handle* h, SweepShape& shape, int block, int* per_sm, int* cl
   for (int cap = 4096; cap >= 1024 && !add(&SweepShape::term_cap, cap); cap /= 2) {
   }
   if (shape.beads_in_smem) add(&SweepShape::rel_in_smem, 1);
-  if (clusters) *clusters = 0;
-  if (clusters && shape.csize > 1) {
-    // the cluster must be schedulable: csize CTAs of this size in one GPC
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = shape.csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(shape.csize);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = SweepSmem::make(shape).total;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(clusters, fn, &cfg);
-    if (e != cudaSuccess || *clusters < 1)
-      return set_error(REMC_ERR_INVALID, "a cluster of %d sweep CTAs does not fit: %s", shape.csize,
-                       cudaGetErrorString(e));
-  }
   return REMC_OK;
 }
 
@@ -1793,22 +1794,31 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
                      h->max_dyn_smem);
   int block = sweep_block(h, threads, (long long)h->n_inst * csize);
   int per_sm = 0, clusters = 0;
-  const int rc = fit_sweep(h, shape, block, &per_sm, &clusters);
+  const int rc = fit_sweep(h, shape, block, &per_sm);
   if (rc) return rc;
-  if (csize > 1 && clusters < h->n_inst && block > 256) {
-    // smaller CTAs where clusters of the larger would run the replicas in waves
-    SweepShape other = base_shape(h, threads, mol_in_smem, csize, beads_in_smem);
-    int n = 0, c = 0;
-    if (!fit_sweep(h, other, 256, &n, &c) && c > clusters) {
-      shape = other;
-      block = 256;
-      per_sm = n;
-      clusters = c;
+  if (csize > 1) {
+    clusters = cluster_room(h, shape, block);
+    if (clusters < h->n_inst && block > 256) {
+      // smaller CTAs where clusters of the larger would run the replicas in waves
+      SweepShape other = base_shape(h, threads, mol_in_smem, csize, beads_in_smem);
+      int n = 0, c = 0;
+      if (!fit_sweep(h, other, 256, &n) && (c = cluster_room(h, other, 256)) > clusters) {
+        shape = other;
+        block = 256;
+        per_sm = n;
+        clusters = c;
+      }
     }
+    if (clusters < 1)
+      return set_error(REMC_ERR_INVALID, "a cluster of %d sweep CTAs does not fit", csize);
   }
   // Replicas fewer than the SMs: a replica of one virtual CTA spreads over a
   // cluster of up to four, each on its own SM, where its chain steps are long
-  // enough (kSpreadPairs) for the cluster barrier they then take.
+  // enough (kSpreadPairs) for the cluster barrier they then take, and all
+  // clusters fit at once: SMs come in GPCs, of which a cluster of four may leave
+  // up to three, so above four fifths of the CTAs the GPU is asked (148 SMs hold
+  // 33 clusters of four CTAs of 512 threads; 34 replicas of 150 + 150 residues
+  // took 2.27 ms per 200 steps in two waves, 1.68 on clusters of two).
   if (csize == 1 && beads_in_smem && h->chain_step_pairs >= kSpreadPairs) {
     for (int c = 4; c > 1; c /= 2) {
       if ((long long)h->n_inst * c > h->num_sms) continue;
@@ -1816,7 +1826,9 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
       wide.vsize = 1;
       wide.aj_in_smem = 1;
       int n = 0;
-      if (SweepSmem::make(wide).total > (size_t)h->max_dyn_smem || fit_sweep(h, wide, block, &n, nullptr))
+      if (SweepSmem::make(wide).total > (size_t)h->max_dyn_smem || fit_sweep(h, wide, block, &n)) continue;
+      if ((long long)h->n_inst * c > (long long)n * h->num_sms * 4 / 5 &&
+          cluster_room(h, wide, block) < h->n_inst)
         continue;
       shape = wide;
       per_sm = n;
@@ -1832,7 +1844,7 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
   if (shape.csize == 1 && beads_in_smem && SweepSmem::make(apart).total <= (size_t)h->max_dyn_smem) {
     choose_apart(h, per_sm * h->num_sms);
     int n = 0;
-    if (h->n_apart && (fit_sweep(h, apart, block, &n, nullptr) || ensure_sweep_scratch(h, apart))) {
+    if (h->n_apart && (fit_sweep(h, apart, block, &n) || ensure_sweep_scratch(h, apart))) {
       h->n_apart = 0;
       h->apart_from = INFINITY;
     }

@@ -46,3 +46,12 @@ def test_cta_sizes(built_lib, chains, crowders, turn, R, threads):
     from remcdockingsimulator_b200.engine import make_params
     s = _system(7, chains, crowders, 6.0, 140.0, turn=turn)
     _check([s], R, make_params(), 40, threads)
+
+
+@pytest.mark.parametrize("R", [29, 30, 33, 34, 37, 60, 74])
+def test_spread_where_clusters_just_fit(built_lib, R):
+    """Replicas of long chain steps about as many as clusters of four and of two
+    CTAs of 512 threads fit at once: the same results wherever they run."""
+    from remcdockingsimulator_b200 import synth
+    s = _system(9, [131, 130], 0, 6.0, 190.0)
+    _check([s], R, synth.benchmark_params(), 12, 256, oracle=R == 34)
