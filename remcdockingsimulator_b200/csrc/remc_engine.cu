@@ -37,6 +37,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <initializer_list>
 #include <mutex>
 #include <string>
@@ -1359,6 +1360,7 @@ struct remc_handle {
   float apart_from = INFINITY;       // expected cost of their systems, at least
   std::vector<float> sys_cost;       // expected cycles per step, by system
   std::vector<float> sys_chain_cost; // of them, in chain steps' pairs
+  std::vector<double> sys_pairs;     // pairs of a chain step, on average
   float* d_sys_cost = nullptr;
   bool all_fold = false;    // every system's fold flag is set (the state uploaded last)
   int nrel = 0;             // beads up to the last one of a molecule of several
@@ -1705,38 +1707,57 @@ constexpr double kOneBeadCycles = 900.0, kOneBeadPairCycles = 1.1;
 // block would otherwise end in their replicas alone: in a batch of unlike
 // systems one with few crowders moves a chain in every third step and takes
 // longer than the whole batch does on average. The prefix of the systems by
-// cost that makes the expected end earliest: the later of the SM slots' mean
-// load and the longest replica, where a cluster takes the chain steps' pairs in
-// a third of the time, all else in 1.2 times it, and four slots. A batch of 64
-// systems ran 15.1 ms per 1000 steps without it (its balanced load is 10.9),
-// 12.3 with four systems apart; every replica on a cluster took 21.9 where
-// none took 15.9.
-void choose_apart(remc_handle* h, int slots) {
+// cost that makes the expected end earliest: the latest of the SM slots' mean
+// load, the clusters, one replica after the other on those that fit at once,
+// and the longest replica of the queue. A cluster takes the chain steps' pairs
+// in a third of the time, all else in 1.2 times it, and four slots; it pays for
+// systems whose chain steps would also have it spread (kSpreadPairs). A batch
+// of 64 systems ran 15.1 ms per 1000 steps without it (its balanced load is
+// 10.9), 12.3 with four systems apart; every replica on a cluster took 21.9
+// where none took 15.9, 76 replicas of 60 + 60 residues 474 us per 60 steps in
+// two waves of clusters where one CTA each takes 250.
+struct Apart {
+  int n = 0;              // instances, the first of the list by cost
+  float from = INFINITY;  // expected cost of their systems, at least
+};
+Apart choose_apart(const remc_handle* h, int slots) {
   std::vector<int> order(h->n_sys);
   for (int q = 0; q < h->n_sys; ++q) order[q] = q;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->sys_cost[a] > h->sys_cost[b]; });
   double load = 0.0;
   for (int q = 0; q < h->n_sys; ++q) load += (double)h->sys_cost[q] * h->h_sys[q].n_rep;
-  double best = 0.9 * std::max(load / slots, (double)h->sys_cost[order[0]]), longest = 0.0;
+  double best = 0.9 * std::max(load / slots, (double)h->sys_cost[order[0]]);
+  // when each cluster is free: a heap, the earliest on top. Clusters of four
+  // leave SMs of a GPC idle: four fifths of the slots are safe
+  const int room = std::max(1, slots / 5);
+  std::vector<double> free_at(room, 0.0);
+  double clusters_end = 0.0;
+  Apart chosen;
   int n = 0;
-  h->n_apart = 0;
-  h->apart_from = INFINITY;
   for (int k = 0; k < h->n_sys; ++k) {
     const int q = order[k];
+    if (h->sys_pairs[q] < kSpreadPairs) break;
     const double t = h->sys_cost[q], c = h->sys_chain_cost[q];
     const double apart = c / 3.3 + 1.2 * (t - c);
-    longest = std::max(longest, apart);
     load += (4.0 * apart - t) * h->h_sys[q].n_rep;
+    for (int r = 0; r < h->h_sys[q].n_rep && clusters_end < best; ++r) {
+      std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
+      free_at.back() += apart;
+      clusters_end = std::max(clusters_end, free_at.back());
+      std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+    }
+    if (clusters_end >= best) break;  // later prefixes end no earlier
     n += h->h_sys[q].n_rep;
     if (k + 1 < h->n_sys && h->sys_cost[order[k + 1]] == h->sys_cost[q]) continue;
     const double rest = k + 1 < h->n_sys ? h->sys_cost[order[k + 1]] : 0.0;
-    const double end = std::max(load / slots, std::max(longest, rest));
+    const double end = std::max(load / slots, std::max(clusters_end, rest));
     if (end < best) {
       best = end;
-      h->n_apart = n;
-      h->apart_from = h->sys_cost[q];
+      chosen.n = n;
+      chosen.from = h->sys_cost[q];
     }
   }
+  return chosen;
 }
 
 // Threads of a sweep CTA, for a schedule of `threads` virtual threads and `ctas`
@@ -1835,23 +1856,22 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
       break;
     }
   }
-  h->sweep_cluster_slots = clusters;
-  h->n_apart = 0;
-  h->apart_from = INFINITY;
+  Apart chosen;
   SweepShape apart = base_shape(h, threads, mol_in_smem, 4, beads_in_smem);
   apart.vsize = 1;
   apart.aj_in_smem = 1;
   if (shape.csize == 1 && beads_in_smem && SweepSmem::make(apart).total <= (size_t)h->max_dyn_smem) {
-    choose_apart(h, per_sm * h->num_sms);
+    chosen = choose_apart(h, per_sm * h->num_sms);
     int n = 0;
-    if (h->n_apart && (fit_sweep(h, apart, block, &n) || ensure_sweep_scratch(h, apart))) {
-      h->n_apart = 0;
-      h->apart_from = INFINITY;
-    }
-    h->apart_shape = apart;
+    if (chosen.n && (fit_sweep(h, apart, block, &n) || ensure_sweep_scratch(h, apart))) chosen = Apart();
   }
   if (ensure_sweep_scratch(h, shape)) return REMC_ERR_NOMEM;
+  // nothing has failed: a schedule is set as a whole
   h->sweep_shape = shape;
+  h->apart_shape = apart;
+  h->n_apart = chosen.n;
+  h->apart_from = chosen.from;
+  h->sweep_cluster_slots = clusters;
   h->sweep_threads = threads;
   h->sweep_block = block;
   h->mol_in_smem = mol_in_smem;
@@ -2143,7 +2163,8 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
       }
       h->any_crowders = h->any_crowders || d.mol_role[m] == -1;
     }
-    if (several) h->chain_step_pairs = std::max(h->chain_step_pairs, pairs / several);
+    h->sys_pairs.push_back(several ? pairs / several : 0.0);
+    h->chain_step_pairs = std::max(h->chain_step_pairs, h->sys_pairs.back());
   }
   if (bead_cursor >= (size_t)1 << 31) {
     delete h;

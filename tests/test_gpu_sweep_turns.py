@@ -55,3 +55,12 @@ def test_spread_where_clusters_just_fit(built_lib, R):
     from remcdockingsimulator_b200 import synth
     s = _system(9, [131, 130], 0, 6.0, 190.0)
     _check([s], R, synth.benchmark_params(), 12, 256, oracle=R == 34)
+
+
+def test_replicas_about_as_many_as_clusters(built_lib):
+    """Between a quarter and half as many replicas as CTAs fit: one CTA each or
+    clusters apart, the same results."""
+    from remcdockingsimulator_b200 import synth
+    for R in (61, 76, 100):
+        s = _system(9, [81, 80], 0, 6.0, 170.0)
+        _check([s], R, synth.benchmark_params(), 16, 128, oracle=False)
