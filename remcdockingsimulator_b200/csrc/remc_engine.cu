@@ -1365,6 +1365,7 @@ struct remc_handle {
   bool all_fold = false;    // every system's fold flag is set (the state uploaded last)
   int nrel = 0;             // beads up to the last one of a molecule of several
   bool any_crowders = false;
+  int crowders_max = 0;     // crowder molecules of a system, at most
   double chain_step_pairs = 0.0;  // pairs of a step of a molecule of several beads, on average
   int num_sms = 148;
   // graph
@@ -1766,24 +1767,27 @@ Apart choose_apart(const remc_handle* h, int slots) {
 // With crowders two warps per virtual warp, 256 or 512: a group of 8 steps then
 // has whole warps or pairs of warps for every step. Without, chain steps only,
 // which all threads share: 512 where a step has pairs for them, 256 for less
-// (100 residues, 20 replicas, 1000 steps: 2.64 ms, 2.79 with 512).
+// (100 residues, 20 replicas, 1000 steps: 2.64 ms, 2.79 with 512; but
+// 100 + 100 residues, 76 replicas, 60 steps: 457 us, 386 with 512).
 //
 // With more CTAs than SMs hold, those wait for whole rounds, and small steps,
 // which are latency, run as fast on fewer threads: half as many, down to 128,
-// where the systems are small. us for 100 steps, 128 / 256 / 512 threads (in
+// where the systems are small or have few crowders, whose groups are short. us
+// for 100 steps, 128 / 256 / 512 threads (in
 // brackets 128 without groups and splits): 20 + 24 residues, 300 replicas 268 /
 // 444 / 685 (353); 100 residues, 1200 replicas 1197 / 1497 / 2482 (1851); 300 +
 // 300 residues, 150 replicas 6062 / 5359 / 7172 (6322); 44 residues and 100
 // crowders, 1200 replicas 304 / 328 / 533 (382); but 100 residues and 400
-// crowders, 600 replicas 243 / 212 / 312 (277).
-constexpr double kWidePairs = 16384.0, kHeavyPairs = 65536.0;
-constexpr int kSmallBeads = 192, kTinyBeads = 96;
+// crowders, 600 replicas 243 / 212 / 312 (277); 290 residues and 18 crowders,
+// 1056 replicas, 256 virtual threads 726 / 887 / 1272 (1202).
+constexpr double kWidePairs = 8192.0, kHeavyPairs = 65536.0;
+constexpr int kSmallBeads = 192, kTinyBeads = 96, kFewCrowders = 32;
 int sweep_block(const remc_handle* h, int threads, long long ctas) {
   const double pairs = h->chain_step_pairs;
   int block, least;
   if (h->any_crowders) {
     block = std::min(kSweepThreads, std::max(256, 2 * threads));
-    least = h->nmax <= kSmallBeads ? 128 : block;
+    least = h->nmax <= kSmallBeads || h->crowders_max <= kFewCrowders ? 128 : block;
   } else {
     block = pairs >= kWidePairs ? kSweepThreads : 256;
     least = pairs < kHeavyPairs ? 128 : 256;
@@ -1819,16 +1823,15 @@ int configure_sweep(remc_handle* h, int threads, int mol_in_smem, int csize, int
   if (rc) return rc;
   if (csize > 1) {
     clusters = cluster_room(h, shape, block);
-    if (clusters < h->n_inst && block > 256) {
-      // smaller CTAs where clusters of the larger would run the replicas in waves
+    // smaller CTAs where clusters of the larger would run the replicas in waves
+    for (int b = block / 2; b >= 128 && clusters < h->n_inst; b /= 2) {
       SweepShape other = base_shape(h, threads, mol_in_smem, csize, beads_in_smem);
       int n = 0, c = 0;
-      if (!fit_sweep(h, other, 256, &n) && (c = cluster_room(h, other, 256)) > clusters) {
-        shape = other;
-        block = 256;
-        per_sm = n;
-        clusters = c;
-      }
+      if (fit_sweep(h, other, b, &n) || (c = cluster_room(h, other, b)) <= clusters) continue;
+      shape = other;
+      block = b;
+      per_sm = n;
+      clusters = c;
     }
     if (clusters < 1)
       return set_error(REMC_ERR_INVALID, "a cluster of %d sweep CTAs does not fit", csize);
@@ -2154,15 +2157,17 @@ int remc_create(const remc_system_desc* systems, int n_systems, const remc_param
     for (int m = 0; m < d.n_mol; ++m)
       if (d.mol_start[m + 1] - d.mol_start[m] > 1) h->nrel = std::max(h->nrel, d.mol_start[m + 1]);
     double pairs = 0.0;
-    int several = 0;
+    int several = 0, crowders = 0;
     for (int m = 0; m < d.n_mol; ++m) {
       const double n = d.mol_start[m + 1] - d.mol_start[m];
       if (n > 1) {
         pairs += n * (d.n_beads - n);
         ++several;
       }
-      h->any_crowders = h->any_crowders || d.mol_role[m] == -1;
+      crowders += d.mol_role[m] == -1;
     }
+    h->any_crowders = h->any_crowders || crowders > 0;
+    h->crowders_max = std::max(h->crowders_max, crowders);
     h->sys_pairs.push_back(several ? pairs / several : 0.0);
     h->chain_step_pairs = std::max(h->chain_step_pairs, h->sys_pairs.back());
   }
