@@ -159,18 +159,6 @@ __device__ __forceinline__ float crowd_energy(float r2, float A, float cut2) {
   return e;
 }
 
-// Change of a crowder pair's energy from squared distance ro to rn: the new
-// energy's last product enters the difference unrounded (written out, so that
-// every caller rounds alike).
-template <bool R12, bool CUT>
-__device__ __forceinline__ float crowd_change(float rn, float ro, float A, float cut2) {
-  if (CUT)
-    return __fsub_rn(crowd_energy<R12, true>(rn, A, cut2), crowd_energy<R12, true>(ro, A, cut2));
-  const float in2 = fast_rcp(rn), in6 = in2 * in2 * in2;
-  const float eo = crowd_energy<R12, false>(ro, A, cut2);
-  return R12 ? __fmaf_rn(A * in6, in6, -eo) : __fmaf_rn(A, in6, -eo);
-}
-
 __device__ __forceinline__ float pair_r2(float4 a, float4 b, float L, float invL) {
   float dx = min_image(a.x - b.x, L, invL);
   float dy = min_image(a.y - b.y, L, invL);
@@ -258,7 +246,9 @@ __device__ __forceinline__ float2 crowd_energy2(float2 r2, float2 A, float2 cut2
   return e;
 }
 
-// crowd_change for two pairs
+// Change of two crowder pairs' energies from squared distances ro to rn: the new
+// energy's last product enters the difference unrounded (written out, so that
+// every caller rounds alike).
 template <bool R12, bool CUT>
 __device__ __forceinline__ float2 crowd_change2(float2 rn, float2 ro, float2 A, float2 cut2) {
   if (CUT) {

@@ -64,3 +64,11 @@ def test_replicas_about_as_many_as_clusters(built_lib):
     for R in (61, 76, 100):
         s = _system(9, [81, 80], 0, 6.0, 170.0)
         _check([s], R, synth.benchmark_params(), 16, 128, oracle=False)
+
+
+def test_clusters_of_small_ctas(built_lib):
+    """More clusters than fit with CTAs of 256 threads: of 128, fewer warps than
+    virtual warps in each."""
+    from remcdockingsimulator_b200.engine import make_params
+    s = _system(7, [20, 24], 12, 6.0, 140.0)
+    _check([s], 45, make_params(), 40, 256, cluster=8)
