@@ -2828,12 +2828,14 @@ int remc_energy_adjoint(remc_handle* h, float* forces, double* mol_force_torque,
                                      h->d_items_by_cost, h->n_items, h->d_adj_queue, h->d_forces,
                                      h->d_G, h->d_dxi, h->d_eadj, consts_of(h), C);
   REMC_CUDA_TRY(cudaGetLastError());
-  if (mol_force_torque) {
+  // what is not asked for is left out; without any output, all is run
+  const bool all = !forces && !mol_force_torque && !dE_dlambda && !dE_dxi && !dE_deps && !energy;
+  if (mol_force_torque || all) {
     molecule_force_torque_kernel<<<dim3(h->n_inst, (h->mmax + 127) / 128), 128, 0, h->stream>>>(
         h->d_sys, h->d_inst_sys, h->d_mol_start, h->d_rel, h->d_forces, h->d_mft);
     REMC_CUDA_TRY(cudaGetLastError());
   }
-  if (dE_deps || dE_dlambda) {
+  if (dE_deps || dE_dlambda || all) {
     deps_kernel<<<h->n_inst, 128, 0, h->stream>>>(h->d_G, h->d_dl, table);
     REMC_CUDA_TRY(cudaGetLastError());
   }
