@@ -1642,7 +1642,7 @@ int ensure_sweep_scratch(remc_handle* h, const SweepShape& p) {
 // A cluster barrier with its remote stores costs some 1,500 cycles a pass, the
 // pairs of a chain step some 0.6 cycles each on one SM: a quarter of them per
 // CTA saves more from about 4,000 pairs on. Two chains of 76 and 24 residues
-// (1,824 pairs): 3.62 ms per 1000 steps spread, 3.15 not (now 2.79); 129 + 57 +
+// (1,824 pairs): 3.62 ms per 1000 steps spread, 3.15 not (now 2.64); 129 + 57 +
 // 201 residues and 233 turning crowders (63,000): 0.80 ms spread, 1.17 not (now
 // 0.66, groups running over the turns).
 constexpr double kSpreadPairs = 4096.0;
